@@ -69,20 +69,20 @@ persistent_loop(PTables& T, Path& p)
         if(wcur >= T.total) { drained = true; wcur = wend = T.total; }
       }
     }
-    if(p.state == ST_IDLE && wcur < wend) path_assign(p, T, wcur++);
+    if(p.state == ST_IDLE && wcur < wend) path_assign(p, p.ri, T, wcur++);
     if(!__any_sync(0xffffffffu, p.state != ST_IDLE)) break;
     if(p.state != ST_IDLE) {
       const DRequest& R = T.reqs[p.ri];
       const DScene& S = T.scenes[p.si];
       if(p.state != ST_TRACE && p.state != ST_DONE) {
-        path_event<V>(p, S, R);
+        path_event<V>(p, p, S, R);
         seg += p.c_seg; node += p.c_node; tc += p.c_tc;
         p.c_seg = p.c_node = p.c_tc = 0;
       }
       if(p.state == ST_TRACE) {
         trace_step<V>(p, S);
       } else if(p.state == ST_DONE) {
-        accumulate_b(p, R);
+        accumulate_b(p, p.weight, R);
         count_grid(T.cnt, p);
         real += (p.flags & (PF_REJECTED | PF_FAILED)) ? 0 : 1;
         fail += (p.flags & PF_FAILED) ? 1 : 0;
@@ -338,9 +338,17 @@ plan_build(Plan& P, const htrdr_gpu_batch_item* items, size_t n, bool host_out,
     acc_off[i] = acc_total;
     acc_total += npix * (nch + 1);
     P.items[i] = PItem{(uint32_t)i, si, 0};
-    P.offsets[i + 1] = P.offsets[i] + npix * P.reqs[i].nreal_pp;
     P.out_off[i] = out_bytes;
     if(host_out) out_bytes += (items[i].layout.pitch * items[i].layout.height + 255) & ~(size_t)255;
+  }
+  /* The work queue takes the shortwave requests first: their walks are tens
+   * of times longer, so the longwave ones fill the lanes that run dry, and
+   * until then a warp's paths are of one kind. */
+  std::stable_partition(P.items.begin(), P.items.end(),
+                        [&](const PItem& it) { return hv_kind(P.reqs[it.req].mode) == HV_SW; });
+  for(size_t k = 0; k < n; ++k) {
+    const DRequest& r = P.reqs[P.items[k].req];
+    P.offsets[k + 1] = P.offsets[k] + (uint64_t)r.width * r.height * r.nreal_pp;
   }
   P.acc_bytes = accum_out ? 0 : acc_total * sizeof(DAccum);
   if((!accum_out && !reserve(B.d_acc, P.acc_bytes)) || !reserve(B.d_cnt, 128) || !reserve(B.d_out, out_bytes))

@@ -5,6 +5,7 @@
 #define HTRDR_DSCENE_H
 
 #include <stdint.h>
+#include <vector_types.h>
 
 #define HG_LEAF 0xFFFFFFFFu
 #define HG_MAX_DIST 1e9f          /* no collision beyond (..._sw.c:118-123) */
@@ -12,6 +13,7 @@
 #define HG_MAX_STEPS (1u << 20)   /* voxel steps per trace before giving up */
 #define HG_MAX_BOUNCES (1u << 16) /* scattering events per realisation before giving up */
 #define HG_MAX_NULL (1u << 22)    /* tentative collisions per voxel before giving up */
+#define HG_LAYER_GUIDE 1024        /* slices of the column in the layer guide */
 #define HG_BVH_DEPTH_MAX 48       /* ground BVH depth bound (the traversal stack size) */
 
 /* Register budget of the transport kernels (per thread): trades occupancy
@@ -76,6 +78,9 @@ struct DScene {
   float ztop;
   const float2* gas;      /* [nq][nlayers] {ka, ks} */
   const double* layer_zd; /* [nlayers+1] layer bounds, FP64 */
+  const uint2* layer_guide; /* [HG_LAYER_GUIDE] layer bounds at or below any height of a slice
+                             * of the column: {fewest, most} */
+  float guide_scale;      /* slices per m */
   const double* gas_cum;  /* [nq][3][nlayers+1] cumulative vertical optical depth from z = 0 */
   /* spectral */
   uint32_t nbands;
@@ -100,6 +105,11 @@ struct DScene {
    * ranks); null unless built instead of leaf_grid */
   const float2* maj_grid;
   const uint8_t* lvl_grid;
+  /* place of cell (x, y, z) in its grid: x gstride[0] + y gstride[1] + z
+   * gstride[2].  maj_flag: the sign of a kmax says that the leaf is larger
+   * than its cell (no majorant of the scene is negative) */
+  uint32_t gstride[3];
+  int32_t maj_flag;
   const uint32_t* grid_rank; /* [nq*3] */
   uint64_t ncell;            /* def[0] * def[1] * def[2] */
   /* ground */

@@ -44,7 +44,7 @@ find_item(const hg::PTables& T, uint64_t g)
  * realisation time, for a path in ST_DONE.  Called by the lanes of a warp
  * whose paths ended, in any subset. */
 __device__ __forceinline__ void
-accumulate_b(const Path& p, const DRequest& R)
+accumulate_b(const PathTrace& p, double weight, const DRequest& R)
 {
   if(R.ndone) atomicAdd(R.ndone, 1ull); /* every realisation, rejected ones included */
   if(p.flags & PF_REJECTED) return;
@@ -60,8 +60,8 @@ accumulate_b(const Path& p, const DRequest& R)
    * pixel apart */
   const cg::coalesced_group here = cg::coalesced_threads();
   const cg::coalesced_group same = cg::labeled_partition(here, (unsigned long long)(uintptr_t)a);
-  const double w = cg::reduce(same, p.weight, cg::plus<double>());
-  const double w2 = cg::reduce(same, p.weight * p.weight, cg::plus<double>());
+  const double w = cg::reduce(same, weight, cg::plus<double>());
+  const double w2 = cg::reduce(same, weight * weight, cg::plus<double>());
   if(same.thread_rank() == 0) {
     atomicAdd(&a->s, w);
     atomicAdd(&a->s2, w2);
@@ -76,8 +76,8 @@ accumulate_b(const Path& p, const DRequest& R)
     atomicAdd(&t->n, (unsigned long long)pix.size());
   }
 #else
-  atomicAdd(&a->s, p.weight);
-  atomicAdd(&a->s2, p.weight * p.weight);
+  atomicAdd(&a->s, weight);
+  atomicAdd(&a->s2, weight * weight);
   atomicAdd(&a->n, 1ull);
   atomicAdd(&t->s, us);
   atomicAdd(&t->s2, us * us);
@@ -88,11 +88,11 @@ accumulate_b(const Path& p, const DRequest& R)
 /* Start realisation `g' (global index) in path p: request, scene, pixel and
  * realisation of the item that holds it */
 __device__ __forceinline__ void
-path_assign(Path& p, const hg::PTables& T, uint64_t g)
+path_assign(PathTrace& p, uint32_t& ri, const hg::PTables& T, uint64_t g)
 {
   const uint32_t ii = find_item(T, g);
   const hg::PItem item = T.items[ii];
-  p.ri = item.req;
+  ri = item.req;
   p.si = item.scene;
   const DRequest& R = T.reqs[item.req];
   const uint64_t local = g - __ldg(T.offsets + ii) + item.begin;
@@ -152,7 +152,7 @@ flush_counts(void* cnt, unsigned long long seg, unsigned long long node, unsigne
 /* Leaf-grid bytes read by a completed path, added to the launch's total: one
  * atomic per realisation, so that no engine keeps another running counter */
 __device__ __forceinline__ void
-count_grid(void* cnt, const Path& p)
+count_grid(void* cnt, const PathTrace& p)
 {
   if(p.c_grid) atomicAdd(&((Counters*)cnt)->grid, (unsigned long long)p.c_grid);
 }
@@ -271,7 +271,7 @@ sorted_loop(hg::PTables& T, PathSlot* slots, uint32_t* lists)
       const bool act = tid < nev;
       Path& p = slots[act ? event_list[tid] : 0].p;
       if(act && p.state == ST_DONE) {
-        accumulate_b(p, T.reqs[p.ri]);
+        accumulate_b(p, p.weight, T.reqs[p.ri]);
         count_grid(T.cnt, p);
         real += (p.flags & (PF_REJECTED | PF_FAILED)) ? 0 : 1;
         fail += (p.flags & PF_FAILED) ? 1 : 0;
@@ -288,12 +288,12 @@ sorted_loop(hg::PTables& T, PathSlot* slots, uint32_t* lists)
         base = __shfl_sync(0xffffffffu, base, leader);
         if(need) {
           const unsigned long long g = base + (unsigned long long)__popc(m & ((1u << lane) - 1u));
-          if(g < T.total) path_assign(p, T, g);
+          if(g < T.total) path_assign(p, p.ri, T, g);
           else n[2] = 1; /* the queue is drained: idle slots stop asking */
         }
       }
       if(act && p.state != ST_IDLE && p.state != ST_TRACE && p.state != ST_DONE) {
-        path_event<V>(p, T.scenes[p.si], T.reqs[p.ri]);
+        path_event<V>(p, p, T.scenes[p.si], T.reqs[p.ri]);
         seg += p.c_seg; node += p.c_node; tc += p.c_tc;
         p.c_seg = p.c_node = p.c_tc = 0;
       }

@@ -118,7 +118,7 @@ void build_octree(const DScene& hs, const float* lwc, const float* sig3, const f
  * grids do not fit or cannot be indexed (the traversal then descends).
  * `majorants': each cell holds its leaf's kmin/kmax (float2, the ntrees x
  * ncell array first) and level (u8, after it) instead of node << 5 | level. */
-bool build_leaf_grids(const DScene& S, const std::vector<uint64_t>& tree_base,
+bool build_leaf_grids(DScene& S, const std::vector<uint64_t>& tree_base,
                       const std::vector<uint64_t>& tree_count, DevBuf& grids, std::vector<uint32_t>& rank,
                       bool majorants);
 

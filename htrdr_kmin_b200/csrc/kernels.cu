@@ -16,7 +16,7 @@ run_path(Path& p, const DScene& S, const DRequest& R)
   for(;;) {
     if(p.state == ST_TRACE) trace_step<V>(p, S);
     else if(p.state == ST_DONE) return;
-    else path_event<V>(p, S, R);
+    else path_event<V>(p, p, S, R);
   }
 }
 

@@ -20,6 +20,7 @@
 
 #include <algorithm>
 #include <cfloat>
+#include <cmath>
 #include <functional>
 #include <memory>
 #include <string>
@@ -172,23 +173,32 @@ k_leafgrid(const uint4* __restrict__ nodes, uint32_t depth, uint32_t nx, uint32_
 
 /* Majorants and level of the leaf of every cell of one tree (the same
  * descent): the trace reads a cell's kmin/kmax and voxel size with two
- * independent loads instead of the grid entry, then the node */
+ * independent loads instead of the grid entry, then the node.  Cells are laid
+ * out by `stride' (ax0 the axis of consecutive entries).  flag: the sign of
+ * kmax marks a leaf larger than a cell, so that a walk through single-cell
+ * leaves needs one load; *negative is set where that sign is taken. */
 __global__ void
-k_majgrid(const uint4* __restrict__ nodes, uint32_t depth, uint32_t nx, uint32_t ny, uint32_t nz,
-          float2* maj, uint8_t* lvl)
+k_majgrid(const uint4* __restrict__ nodes, uint32_t depth, uint3 def, uint32_t ax0, uint32_t ax1, int flag,
+          float2* maj, uint8_t* lvl, int* negative)
 {
   const uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if(c >= (uint64_t)nx * ny * nz) return;
-  const uint32_t x = (uint32_t)(c % nx), y = (uint32_t)((c / nx) % ny), z = (uint32_t)(c / ((uint64_t)nx * ny));
-  uint32_t n = 0, L = depth;
+  const uint32_t n[3] = {def.x, def.y, def.z};
+  if(c >= (uint64_t)n[0] * n[1] * n[2]) return;
+  const uint32_t n0 = n[ax0], n1 = n[ax1], ax2 = 3u - ax0 - ax1;
+  uint32_t at[3];
+  at[ax0] = (uint32_t)(c % n0);
+  at[ax1] = (uint32_t)((c / n0) % n1);
+  at[ax2] = (uint32_t)(c / ((uint64_t)n0 * n1));
+  uint32_t i = 0, L = depth;
   uint32_t child = nodes[0].z;
   while(child != HG_LEAF && L > 0) {
     --L;
-    n = child + (((x >> L) & 1u) | (((y >> L) & 1u) << 1) | (((z >> L) & 1u) << 2));
-    child = nodes[n].z;
+    i = child + (((at[0] >> L) & 1u) | (((at[1] >> L) & 1u) << 1) | (((at[2] >> L) & 1u) << 2));
+    child = nodes[i].z;
   }
-  const uint4 v = nodes[n];
-  maj[c] = make_float2(__uint_as_float(v.x), __uint_as_float(v.y));
+  const uint4 v = nodes[i];
+  if((int)v.y < 0) *negative = 1;
+  maj[c] = make_float2(__uint_as_float(v.x), __uint_as_float(flag && L ? v.y | 0x80000000u : v.y));
   lvl[c] = (uint8_t)L;
 }
 
@@ -199,7 +209,7 @@ k_majgrid(const uint4* __restrict__ nodes, uint32_t depth, uint32_t nx, uint32_t
  * error) when they would not fit in half of the free device memory or a tree
  * is too large for the 27-bit node index of an entry. */
 bool
-build_leaf_grids(const DScene& S, const std::vector<uint64_t>& tree_base,
+build_leaf_grids(DScene& S, const std::vector<uint64_t>& tree_base,
                  const std::vector<uint64_t>& tree_count, DevBuf& grids, std::vector<uint32_t>& rank,
                  bool majorants)
 {
@@ -217,20 +227,44 @@ build_leaf_grids(const DScene& S, const std::vector<uint64_t>& tree_base,
   const uint64_t bytes = (uint64_t)ntrees * ncell * (majorants ? 9 : 4);
   if(bytes > free_b / 2) return false;
   if(!grids.alloc(bytes)) return false;
-  for(size_t i = 0; i < tree_count.size(); ++i) {
-    if(!tree_count[i]) continue;
-    const uint64_t off = (uint64_t)rank[i] * ncell;
-    if(majorants) {
-      float2* maj = (float2*)grids.ptr;
-      uint8_t* lvl = (uint8_t*)(maj + (uint64_t)ntrees * ncell);
-      k_majgrid<<<grid_of(ncell, 256), 256>>>(S.nodes + tree_base[i], S.depth, S.def[0], S.def[1],
-                                               S.def[2], maj + off, lvl + off);
-    } else {
-      k_leafgrid<<<grid_of(ncell, 256), 256>>>(S.nodes + tree_base[i], S.depth, S.def[0], S.def[1],
-                                                S.def[2], (uint32_t*)grids.ptr + off);
-    }
+  if(!majorants) {
+    for(size_t i = 0; i < tree_count.size(); ++i)
+      if(tree_count[i])
+        k_leafgrid<<<grid_of(ncell, 256), 256>>>(S.nodes + tree_base[i], S.depth, S.def[0], S.def[1], S.def[2],
+                                                  (uint32_t*)grids.ptr + (uint64_t)rank[i] * ncell);
+    return cuda_ok(cudaGetLastError(), "leaf grids") && cuda_ok(cudaDeviceSynchronize(), "leaf grids");
   }
-  return cuda_ok(cudaGetLastError(), "leaf grids") && cuda_ok(cudaDeviceSynchronize(), "leaf grids");
+  /* most voxels of a cloudy scene are crossed by rays towards the sun, so the
+   * axis whose faces these cross most often holds the consecutive entries
+   * (four cells of it in one 32-byte sector); then x, y, z in order */
+  uint32_t ax0 = 2;
+  double most = -1.0;
+  for(uint32_t a = 0; a < 3; ++a) {
+    const double r = std::fabs(S.sun_dir_d[a]) * (double)S.inv_cell[a];
+    if(r > most) { most = r; ax0 = a; }
+  }
+  const uint32_t ax1 = ax0 == 0 ? 1 : 0, ax2 = 3 - ax0 - ax1;
+  S.gstride[ax0] = 1;
+  S.gstride[ax1] = S.def[ax0];
+  S.gstride[ax2] = S.def[ax0] * S.def[ax1];
+  DevBuf neg;
+  if(!neg.alloc(sizeof(int)) || !cuda_ok(cudaMemset(neg.ptr, 0, sizeof(int)), "memset")) return false;
+  float2* maj = (float2*)grids.ptr;
+  uint8_t* lvl = (uint8_t*)(maj + (uint64_t)ntrees * ncell);
+  for(S.maj_flag = ncell < (1ull << 32) ? 1 : 0;; S.maj_flag = 0) {
+    for(size_t i = 0; i < tree_count.size(); ++i) {
+      if(!tree_count[i]) continue;
+      const uint64_t off = (uint64_t)rank[i] * ncell;
+      k_majgrid<<<grid_of(ncell, 256), 256>>>(S.nodes + tree_base[i], S.depth,
+                                               make_uint3(S.def[0], S.def[1], S.def[2]), ax0, ax1, S.maj_flag,
+                                               maj + off, lvl + off, (int*)neg.ptr);
+    }
+    int negative = 0;
+    if(!cuda_ok(cudaGetLastError(), "leaf grids")
+    || !cuda_ok(cudaMemcpy(&negative, neg.ptr, sizeof(int), cudaMemcpyDeviceToHost), "leaf grids"))
+      return false;
+    if(!negative || !S.maj_flag) return true;
+  }
 }
 
 /* Scratch and stream of one build worker: the level arrays of one tree, the

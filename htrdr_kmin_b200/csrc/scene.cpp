@@ -750,6 +750,37 @@ scene_create(int device, const htrdr_gpu_scene_desc* desc, const char* cache_pat
   S.nlayers = nl;
   S.ztop = lz[nl];
   S.nbands = nb;
+  { /* sun (src/atmosphere/htrdr_atmosphere_sun.c:66-101) */
+    const double pi = 3.14159265358979323846;
+    const double az = desc->sun_azimuth * pi / 180.0, el = desc->sun_elevation * pi / 180.0;
+    double d[3] = {std::cos(el) * std::cos(az), std::cos(el) * std::sin(az), std::sin(el)};
+    double b1[3], b2[3];
+    onb_d(d, b1, b2);
+    for(int i = 0; i < 3; ++i) {
+      S.sun_dir_d[i] = d[i];
+      S.sun_dir[i] = (float)d[i];
+      S.sun_b1[i] = (float)b1[i];
+      S.sun_b2[i] = (float)b2[i];
+    }
+    S.sun_cos_half = std::cos(4.6524e-3);
+    S.sun_solid_angle = 2.0 * pi * (1.0 - S.sun_cos_half);
+    S.sun_T = 5778.0;
+  }
+  /* layer guide: the slice of a height is found in single precision, hence
+   * the slack at its ends */
+  std::vector<uint2> guide(HG_LAYER_GUIDE);
+  S.guide_scale = S.ztop > 0.f ? (float)HG_LAYER_GUIDE / S.ztop : 0.f;
+  for(uint32_t i = 0; i < HG_LAYER_GUIDE; ++i) {
+    const double slack = 1e-5 * (double)S.ztop;
+    const double zlo = (double)S.ztop * i / HG_LAYER_GUIDE - slack;
+    const double zhi = (double)S.ztop * (i + 1) / HG_LAYER_GUIDE + slack;
+    const double* z = desc->layer_z;
+    guide[i].x = (uint32_t)(std::upper_bound(z, z + nl + 1, zlo) - z);
+    guide[i].y = i + 1 == HG_LAYER_GUIDE ? nl + 1 : (uint32_t)(std::upper_bound(z, z + nl + 1, zhi) - z);
+    if(!(S.ztop > 0.f)) guide[i] = make_uint2(0, nl + 1);
+  }
+  if(!(S.layer_guide = (const uint2*)upload(guide.data(), guide.size() * sizeof(uint2))))
+    return HTRDR_GPU_RES_MEM_ERR;
   if(!(S.layer_zd = (const double*)upload(desc->layer_z, (nl + 1) * 8))
   || !(S.gas_cum = (const double*)upload(cum_tau.data(), cum_tau.size() * 8))
   || !(S.layer_z = (const float*)upload(lz.data(), lz.size() * 4))
@@ -938,22 +969,6 @@ scene_create(int device, const htrdr_gpu_scene_desc* desc, const char* cache_pat
   {
     const htrdr_gpu_res_T res = setup_ground_mesh(desc, S, upload);
     if(res != HTRDR_GPU_RES_OK) return res;
-  }
-  { /* sun (src/atmosphere/htrdr_atmosphere_sun.c:66-101) */
-    const double pi = 3.14159265358979323846;
-    const double az = desc->sun_azimuth * pi / 180.0, el = desc->sun_elevation * pi / 180.0;
-    double d[3] = {std::cos(el) * std::cos(az), std::cos(el) * std::sin(az), std::sin(el)};
-    double b1[3], b2[3];
-    onb_d(d, b1, b2);
-    for(int i = 0; i < 3; ++i) {
-      S.sun_dir_d[i] = d[i];
-      S.sun_dir[i] = (float)d[i];
-      S.sun_b1[i] = (float)b1[i];
-      S.sun_b2[i] = (float)b2[i];
-    }
-    S.sun_cos_half = std::cos(4.6524e-3);
-    S.sun_solid_angle = 2.0 * pi * (1.0 - S.sun_cos_half);
-    S.sun_T = 5778.0;
   }
   if(!cuda_ok(cudaStreamCreateWithFlags(&scn->stream, cudaStreamNonBlocking), "cudaStreamCreate"))
     return HTRDR_GPU_RES_BAD_OP;

@@ -101,11 +101,24 @@ __device__ __forceinline__ float3 mk3(float x, float y, float z) { return make_f
 __device__ __forceinline__ float3 add3(float3 a, float3 b) { return mk3(a.x + b.x, a.y + b.y, a.z + b.z); }
 __device__ __forceinline__ float3 mul3(float3 a, float s) { return mk3(a.x * s, a.y * s, a.z * s); }
 __device__ __forceinline__ float3 neg3(float3 a) { return mk3(-a.x, -a.y, -a.z); }
-__device__ __forceinline__ float dot3(float3 a, float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+/* Sums of products are written out with their fused operations: which product
+ * is rounded must not depend on the code around an inlined call, or the same
+ * path would take other steps in another kernel. */
+__device__ __forceinline__ float
+sum2(float a, float b, float c, float d) { return fmaf(a, b, __fmul_rn(c, d)); }
+__device__ __forceinline__ float
+dot3(float3 a, float3 b) { return fmaf(a.z, b.z, sum2(a.x, b.x, a.y, b.y)); }
 __device__ __forceinline__ float3 nrm3(float3 a) { return mul3(a, rsqrtf(dot3(a, a))); }
 __device__ __forceinline__ float3 madd3(float3 o, float3 d, float t)
 {
   return mk3(fmaf(d.x, t, o.x), fmaf(d.y, t, o.y), fmaf(d.z, t, o.z));
+}
+/* Mirror direction of wo about N */
+__device__ __forceinline__ float3
+reflect3(float3 n, float3 wo)
+{
+  const float c = 2.f * fmaf(n.z, wo.z, sum2(n.y, wo.y, n.x, wo.x));
+  return nrm3(mk3(fmaf(n.x, c, -wo.x), fmaf(n.y, c, -wo.y), fmaf(n.z, c, -wo.z)));
 }
 __device__ __forceinline__ float comp(float3 v, int a) { return a == 0 ? v.x : (a == 1 ? v.y : v.z); }
 
@@ -129,7 +142,10 @@ around(float3 axis, float mu, float u)
   const float s = sqrtf(fmaxf(0.f, 1.f - mu * mu));
   onb(axis, b1, b2);
   sincospif(2.f * u, &sp, &cp);
-  return nrm3(add3(add3(mul3(b1, cp * s), mul3(b2, sp * s)), mul3(axis, mu)));
+  cp = __fmul_rn(cp, s);
+  sp = __fmul_rn(sp, s);
+  return nrm3(mk3(fmaf(axis.x, mu, sum2(b1.x, cp, b2.x, sp)), fmaf(axis.y, mu, sum2(b1.y, cp, b2.y, sp)),
+                  fmaf(axis.z, mu, sum2(b1.z, cp, b2.z, sp))));
 }
 
 /*******************************************************************************
@@ -437,6 +453,7 @@ struct Trace {
   uint32_t p_base, g_base;
   uint8_t p_level, g_level, start;
   uint8_t kind, prop, region, has_cloud, hit, event;
+  uint8_t enter;           /* the current region is not set up yet (trace_enter) */
 };
 
 /*******************************************************************************
@@ -458,10 +475,11 @@ struct Counters {
   unsigned long long seg, node, tc, real, fail, grid;
 };
 
-struct Path {
-  /* trace part: everything trace_step reads or writes.  It comes first so
-   * that the wavefront engine's trace stage moves only this prefix of a
-   * stored path (HG_TRACE_WORDS). */
+/* Trace part of a path: everything trace_step reads or writes, and the walk
+ * fields the wavefront's trace stage touches when it runs a LW scattering
+ * itself.  It comes first so that the trace stage moves only this prefix of a
+ * stored path. */
+struct PathTrace {
   Rng rng;
   uint32_t c_grid;      /* local counter of leaf-grid bytes read (the word before
                          * the 8-byte aligned Trace: no extra storage) */
@@ -471,12 +489,13 @@ struct Path {
   unsigned long long t0;
   uint32_t c_seg, c_node, c_tc; /* local counters */
   uint8_t state, ret, mode, chan;
-  /* walk fields the wavefront's trace stage reads or writes when it runs a
-   * LW scattering itself, and the realisation's pixel and index */
   uint32_t bounces;
   float gdist;          /* ground distance along the current free path, < 0: none */
-  uint32_t pix, ireal;
-  /* event part */
+  uint32_t pix, ireal;  /* the realisation's pixel and index */
+};
+
+/* Event part: read and written between traces only */
+struct PathEvent {
   float3 org, rdir;     /* sensor ray */
   float3 pos, dir, pnext, dnext, sdir;
   double w, wdirect, inv_pdf, L_sun, weight, wlen_d;
@@ -489,11 +508,10 @@ struct Path {
   uint8_t gedge, prev_edge;
 };
 
-/* 32-bit words of a stored path, and of its trace part */
-#define HG_PATH_WORDS ((uint32_t)(sizeof(Path) / 4))
-#define HG_TRACE_WORDS ((uint32_t)(offsetof(Path, org) / 4))
-static_assert(offsetof(Path, tr) == 40 && offsetof(Path, org) == 240, "trace prefix of 15 vectors");
-static_assert(sizeof(Path) % 4 == 0 && offsetof(Path, org) % 4 == 0, "word-wise path storage");
+struct Path : PathTrace, PathEvent {};
+
+static_assert(offsetof(PathTrace, tr) == 40 && sizeof(PathTrace) == 240, "trace prefix of 15 vectors");
+static_assert(sizeof(Path) == sizeof(PathTrace) + sizeof(PathEvent), "a stored path is its two parts");
 
 __device__ __forceinline__ unsigned long long
 gtimer()
@@ -534,99 +552,130 @@ region_bounds(const Trace& T, int r, float& s, float& e, bool& cloud)
   else { s = T.cb1; e = T.tb; cloud = false; }
 }
 
-/* Set up the current region (skipping empty ones) at its start */
+/* Past the empty regions (the cloud region of a trace that has one is never
+ * empty) */
 __device__ __forceinline__ void
-region_enter(Trace& T, const DScene& S)
+region_skip(Trace& T)
 {
-  const int nreg = T.has_cloud ? 3 : 1;
-  while(T.region < nreg) {
-    float s, e;
-    bool cloud;
-    region_bounds(T, T.region, s, e, cloud);
-    if(s < e) {
-      T.t = s;
-      const float3 p = madd3(T.o, T.d, s);
-      if(!cloud) {
-        int l = layer_of(S, p.z);
-        if(T.d.z < 0.f && l > 0 && p.z <= __ldg(S.layer_z + l)) --l;
-        T.layer = l;
-      } else {
-#pragma unroll
-        for(int a = 0; a < 3; ++a) {
-          int g = __float2int_rd((comp(p, a) - S.lower[a]) * S.inv_cell[a]);
-          if(S.repeat && a < 2) {
-            const int tl = floordiv_i(g, (int)S.def[a]);
-            T.tile[a] = tl;
-            g -= tl * (int)S.def[a];
-          }
-          g = max(0, min(g, (int)S.def[a] - 1));
-          T.c[a] = (uint32_t)g;
-        }
-        if(!S.repeat) { T.tile[0] = 0; T.tile[1] = 0; }
-        T.start = 0; /* descend from the root */
-      }
-      return;
-    }
-    ++T.region;
-  }
+  if(!T.has_cloud) return;
+  if(T.region == 0 && !(T.ta < T.cb0)) T.region = 1;
+  if(T.region == 2 && !(T.cb1 < T.tb)) T.region = 3;
 }
 
+/* Set up the region a trace just came to.  It runs at the region's first
+ * voxel and not where the last one ended, so that a kernel holds one copy of
+ * it: the walk's code, run once per bounce from end to end, is larger than
+ * the instruction cache. */
 __device__ __forceinline__ void
-trace_begin(Path& p, const DScene& S, int kind, int prop, float3 o, float3 d, float t0,
-            float t1, uint8_t ret)
+trace_enter(Trace& T, const DScene& S)
+{
+  if(!T.enter) return;
+  T.enter = 0;
+  const int nreg = T.has_cloud ? 3 : 1;
+  if(T.region >= nreg) return;
+  float s, e;
+  bool cloud;
+  region_bounds(T, T.region, s, e, cloud);
+  T.t = s;
+  const float3 p = madd3(T.o, T.d, s);
+  if(!cloud) {
+    /* only a horizontal ray walks layer by layer (trace_voxel): any other
+     * takes the region in one step (gas_region) */
+    if(T.d.z == 0.f) T.layer = layer_of(S, p.z);
+    return;
+  }
+  T.tile[0] = T.tile[1] = 0;
+#pragma unroll
+  for(int a = 0; a < 3; ++a) {
+    const int n = (int)S.def[a];
+    int g = __float2int_rd((comp(p, a) - S.lower[a]) * S.inv_cell[a]);
+    if(a < 2 && (uint32_t)g >= (uint32_t)n && S.repeat) {
+      const int tl = floordiv_i(g, n);
+      T.tile[a] = tl;
+      g -= tl * n;
+    }
+    T.c[a] = (uint32_t)max(0, min(g, n - 1));
+  }
+  T.start = 0; /* descend from the root */
+}
+
+/* What a trace is asked: one is begun in a single place of each kernel */
+struct TraceArgs {
+  int kind, prop;
+  uint8_t ret;
+  float3 o, d;
+  float t1; /* from 0 to here along the ray */
+};
+
+__device__ __forceinline__ void
+trace_begin(PathTrace& p, const DScene& S, const TraceArgs& q)
 {
   Trace& T = p.tr;
-  T.kind = (uint8_t)kind;
-  T.prop = (uint8_t)prop;
-  T.o = o;
-  T.d = d;
-  T.inv = mk3(1.f / d.x, 1.f / d.y, 1.f / d.z);
+  T.kind = (uint8_t)q.kind;
+  T.prop = (uint8_t)q.prop;
+  T.o = q.o;
+  T.d = q.d;
+  T.inv = mk3(1.f / q.d.x, 1.f / q.d.y, 1.f / q.d.z);
   T.hit = 0;
   T.event = 2;
   T.Tmin = 0.0;
   T.tcur = 0.f;
   T.steps = 0;
   T.region = 0;
-  if(kind == TK_TRANS) {
+  T.enter = 1;
+  T.Ts = p.rng.exp1(); /* ..._sw.c:239, :353, ..._lw.c:193 */
+  if(q.kind != TK_TRANS) {
     /* a transmissivity trace sets no collision site: the site of the free
      * path before it stays for the scattering that follows (the absorption
      * transmissivity to a collision site, ..._sw.c:394-398) */
-    T.Ts = p.rng.exp1(); /* ..._sw.c:239 */
-  } else {
     T.site_cell = -1;
     T.site_layer = -1;
   }
   p.state = ST_TRACE;
-  p.ret = ret;
+  p.ret = q.ret;
 
-  float ta = t0, tb = fminf(t1, HG_MAX_DIST);
-  slab(o.z, d.z, T.inv.z, 0.f, S.ztop, ta, tb);
+  float ta = 0.f, tb = fminf(q.t1, HG_MAX_DIST);
+  slab(q.o.z, q.d.z, T.inv.z, 0.f, S.ztop, ta, tb);
   T.ta = ta; T.tb = tb;
   T.has_cloud = 0;
   if(!(ta < tb)) { T.region = 3; T.ta = T.tb = 0.f; return; }
   if(S.has_cloud) {
     float c0 = ta, c1 = tb;
     if(!S.repeat) {
-      slab(o.x, d.x, T.inv.x, S.lower[0], S.upper[0], c0, c1);
-      slab(o.y, d.y, T.inv.y, S.lower[1], S.upper[1], c0, c1);
+      slab(q.o.x, q.d.x, T.inv.x, S.lower[0], S.upper[0], c0, c1);
+      slab(q.o.y, q.d.y, T.inv.y, S.lower[1], S.upper[1], c0, c1);
     }
-    slab(o.z, d.z, T.inv.z, S.lower[2], S.upper[2], c0, c1);
+    slab(q.o.z, q.d.z, T.inv.z, S.lower[2], S.upper[2], c0, c1);
     if(c0 < c1) {
       T.has_cloud = 1;
       T.cb0 = c0;
       T.cb1 = c1;
-      T.base = S.tree_base[(size_t)p.q * 3 + prop];
-      T.grank = S.grid_rank ? __ldg(S.grid_rank + (size_t)p.q * 3 + prop) : 0u;
+      if(!S.maj_grid) T.base = S.tree_base[(size_t)p.q * 3 + q.prop]; /* no node is read through the grid */
+      T.grank = S.grid_rank ? __ldg(S.grid_rank + (size_t)p.q * 3 + q.prop) : 0u;
+      region_skip(T);
     }
   }
-  region_enter(T, S);
+}
+
+/* Gas layer of a point at height z in a cloud cell of z index `kz': clamped
+ * into the layers the cell overlaps (no search where it overlaps one) */
+__device__ __forceinline__ int
+cell_layer(const DScene& S, int kz, float z)
+{
+  const int2 lr = __ldg(S.cell_layers + kz);
+  if(lr.x < 0) return -1;
+  if(lr.x == lr.y) return lr.x;
+  return max(lr.x, min(layer_of(S, z), lr.y));
 }
 
 /* Collision site (cell clamped into the voxel box, gas layer clamped into the
  * layers the cell overlaps) of a point inside the current voxel. */
+struct Voxel {
+  uint32_t lo[3], hi[3];
+};
+
 __device__ __forceinline__ void
-site_of(const DScene& S, const Trace& T, bool cloud, const uint32_t lo[3], const uint32_t hi[3],
-        float3 x, int& cell, int& layer)
+site_of(const DScene& S, const Trace& T, bool cloud, const Voxel& vx, float3 x, int& cell, int& layer)
 {
   if(!cloud) { cell = -1; layer = T.layer; return; }
   int c[3];
@@ -634,20 +683,26 @@ site_of(const DScene& S, const Trace& T, bool cloud, const uint32_t lo[3], const
   for(int a = 0; a < 3; ++a) {
     int g = __float2int_rd((comp(x, a) - S.lower[a]) * S.inv_cell[a]);
     if(a < 2) g -= T.tile[a] * (int)S.def[a];
-    c[a] = max((int)lo[a], min(g, (int)hi[a] - 1));
+    c[a] = max((int)vx.lo[a], min(g, (int)vx.hi[a] - 1));
   }
   cell = (c[2] * (int)S.def[1] + c[1]) * (int)S.def[0] + c[0];
-  const int2 lr = __ldg(S.cell_layers + c[2]);
-  if(lr.x < 0) { layer = -1; return; }
-  layer = max(lr.x, min(layer_of(S, x.z), lr.y));
+  layer = cell_layer(S, c[2], x.z);
+}
+
+/* Optical depth ts less the one over a length l at k.  One rounding: every
+ * engine must walk through the same sums. */
+__device__ __forceinline__ double
+sub_tau(double ts, double l, double k)
+{
+  return fma(-l, k, ts);
 }
 
 /* The hit filters (..._sw.c:73-217, ..._lw.c:64-135) on voxel [d0, d1].
  * Returns true when the traversal stops (real collision). */
 template <unsigned V>
 __device__ __forceinline__ bool
-voxel_filter(Path& p, const DScene& S, float d0, float d1, float kmin, float kmax, bool cloud,
-             const uint32_t lo[3], const uint32_t hi[3])
+voxel_filter(PathTrace& p, const DScene& S, float d0, float d1, float kmin, float kmax, bool cloud,
+             const Voxel& vx)
 {
   Trace& T = p.tr;
   /* the kinds the variant can meet (a LW-only variant meets TK_LW alone) */
@@ -657,56 +712,66 @@ voxel_filter(Path& p, const DScene& S, float d0, float d1, float kmin, float kma
    * free paths still advance it far from the origin */
   double tc = (double)d0;
   const double e = (double)d1;
+  double kt = (double)kmax; /* free paths are sampled against kmax, null ones against kmax - kmin */
   if(trans) {
-    T.Tmin += (e - tc) * (double)kmin;
+    T.Tmin = fma(e - tc, (double)kmin, T.Tmin);
     if(T.Tmin >= HG_TMIN_ZERO) return true; /* exp(-Tmin) is already 0.0 */
-    const double kdif = (double)kmax - (double)kmin;
-    for(uint32_t it = 0;; ++it) {
-      const double Tdif = (e - tc) * kdif;
-      if(T.Ts > Tdif) { T.Ts -= Tdif; T.tcur = d1; return false; }
-      if(it >= HG_MAX_NULL) { p.flags |= PF_FAILED; return true; }
-      tc += T.Ts / kdif;
-      T.tcur = (float)tc;
-      int cell, layer;
-      site_of(S, T, cloud, lo, hi, madd3(T.o, T.d, T.tcur), cell, layer);
+    kt -= (double)kmin;
+  }
+  for(uint32_t it = 0;; ++it) {
+    const double l = e - tc;
+    if(T.Ts > __dmul_rn(l, kt)) { T.Ts = sub_tau(T.Ts, l, kt); T.tcur = d1; return false; }
+    if(it >= HG_MAX_NULL) { p.flags |= PF_FAILED; if(!trans) T.tcur = d1; return trans; }
+    tc += T.Ts / kt;
+    T.tcur = (float)tc;
+    if(!trans && tc > (double)HG_MAX_DIST) return false;
+    int cell, layer;
+    site_of(S, T, cloud, vx, madd3(T.o, T.d, T.tcur), cell, layer);
+    ++p.c_tc;
+    const float r = p.rng.uf();
+    if(trans) {
       float k = site_k(S, cell, layer, p.band, p.q, T.prop, 3);
       k = fminf(fmaxf(k, kmin), kmax);
-      ++p.c_tc;
-      if((double)p.rng.uf() < ((double)k - (double)kmin) / kdif) return true;
-      T.Ts = p.rng.exp1();
-    }
-  } else {
-    for(uint32_t it = 0;; ++it) {
-      const double Tv = (e - tc) * (double)kmax;
-      if(T.Ts > Tv) { T.Ts -= Tv; T.tcur = d1; return false; }
-      if(it >= HG_MAX_NULL) { p.flags |= PF_FAILED; T.tcur = d1; return false; }
-      tc += T.Ts / (double)kmax;
-      T.tcur = (float)tc;
-      if(tc > (double)HG_MAX_DIST) return false;
-      int cell, layer;
-      site_of(S, T, cloud, lo, hi, madd3(T.o, T.d, T.tcur), cell, layer);
-      ++p.c_tc;
+      if((double)r < ((double)k - (double)kmin) / kt) return true;
+    } else {
+      const float ks = site_k(S, cell, layer, p.band, p.q, HG_KS, 3);
+      const float ps = ks / kmax;
+      int event = 2;
       if(scat) {
-        const float ks = site_k(S, cell, layer, p.band, p.q, HG_KS, 3);
-        if(p.rng.uf() < ks / kmax) { T.site_cell = cell; T.site_layer = layer; return true; }
+        if(r < ps) event = T.event; /* a scattering: the event field is the LW walk's */
+        else event = 3;
       } else {
         const float ka = site_k(S, cell, layer, p.band, p.q, HG_KA, 3);
-        const float ks = site_k(S, cell, layer, p.band, p.q, HG_KS, 3);
-        const float r = p.rng.uf();
-        const float pa = ka / kmax, ps = ks / kmax;
-        if(r < pa) { T.event = 0; T.site_cell = cell; T.site_layer = layer; return true; }
-        if(r < pa + ps) { T.event = 1; T.site_cell = cell; T.site_layer = layer; return true; }
+        const float pa = ka / kmax;
+        event = r < pa ? 0 : (r < pa + ps ? 1 : 3);
       }
-      T.Ts = p.rng.exp1();
+      if(event != 3) {
+        T.event = (uint8_t)event;
+        T.site_cell = cell;
+        T.site_layer = layer;
+        return true;
+      }
     }
+    T.Ts = p.rng.exp1();
   }
 }
 
 __device__ __forceinline__ void
-trace_finish(Path& p, bool hit)
+trace_finish(PathTrace& p, bool hit)
 {
   p.tr.hit = hit ? 1 : 0;
   p.state = p.ret;
+}
+
+/* The current region ends, and after the last one the trace */
+__device__ __forceinline__ void
+region_leave(PathTrace& p)
+{
+  Trace& T = p.tr;
+  ++T.region;
+  region_skip(T);
+  T.enter = 1;
+  if(T.region >= (T.has_cloud ? 3 : 1)) trace_finish(p, false);
 }
 
 /* SW walk after a free path that ended by a collision in the medium: the
@@ -715,13 +780,11 @@ trace_finish(Path& p, bool hit)
  * part of the path, so the wavefront's trace stage runs it in place of an
  * event-stage visit.  Returns the collision site (pos_next). */
 __device__ __forceinline__ float3
-sw_scat_volume(Path& p, const DScene& S)
+sw_scat_volume(PathTrace& p, TraceArgs& q)
 {
-  const float3 o = p.tr.o, d = p.tr.d;
-  const float tdst = p.tr.tcur;
+  q = TraceArgs{TK_TRANS, HG_KA, ST_SW_ABS_END, p.tr.o, p.tr.d, p.tr.tcur};
   p.flags &= ~(PF_SURFACE | PF_PREV_GROUND);
-  trace_begin(p, S, TK_TRANS, HG_KA, o, d, 0.f, tdst, ST_SW_ABS_END);
-  return madd3(o, d, tdst);
+  return madd3(q.o, q.d, q.t1);
 }
 
 /* Vertical optical depth from z = 0 to z (clamped to the column) */
@@ -729,7 +792,10 @@ __device__ __forceinline__ double
 gas_tau_at(const DScene& S, const double* cum, uint32_t q, int prop, double z)
 {
   z = fmin(fmax(z, 0.0), (double)S.ztop);
-  uint32_t lo = 0, hi = S.nlayers + 1; /* upper bound on the FP64 bounds */
+  /* bounds <= z, between the guide's two: the same but for a slice that holds
+   * a bound, so no load of the search's six dependent ones most often */
+  const uint2 g = __ldg(S.layer_guide + min((int)((float)z * S.guide_scale), HG_LAYER_GUIDE - 1));
+  uint32_t lo = g.x, hi = g.y;
   while(lo < hi) {
     const uint32_t mid = (lo + hi) >> 1;
     if(__ldg(S.layer_zd + mid) <= z) lo = mid + 1; else hi = mid;
@@ -749,7 +815,7 @@ gas_tau_at(const DScene& S, const double* cum, uint32_t q, int prop, double z)
  * the trace stops (real collision). */
 template <unsigned V>
 __device__ __forceinline__ bool
-gas_region(Path& p, const DScene& S, float re)
+gas_region(PathTrace& p, const DScene& S, float re)
 {
   Trace& T = p.tr;
   const bool trans = (V & HV_SW) && T.kind == TK_TRANS;
@@ -808,10 +874,10 @@ gas_region(Path& p, const DScene& S, float re)
   }
 }
 
-/* One voxel of the current trace */
+/* One voxel of the current trace, its region set up */
 template <unsigned V>
 __device__ __forceinline__ void
-trace_step(Path& p, const DScene& S)
+trace_voxel(PathTrace& p, const DScene& S)
 {
   Trace& T = p.tr;
   const int nreg = T.has_cloud ? 3 : 1;
@@ -823,115 +889,103 @@ trace_step(Path& p, const DScene& S)
   ++p.c_seg;
   if(!cloud && T.d.z != 0.f) { /* the whole gas region at once */
     if(gas_region<V>(p, S, re)) { trace_finish(p, true); return; }
-    ++T.region;
-    region_enter(T, S);
+    region_leave(p);
     return;
   }
-  if(!cloud) {
-    const int l = T.layer;
-    float tn = FLT_MAX;
-    if(T.d.z > 0.f) tn = (__ldg(S.layer_z + l + 1) - T.o.z) * T.inv.z;
-    else if(T.d.z < 0.f) tn = (__ldg(S.layer_z + l) - T.o.z) * T.inv.z;
-    const float t1 = fmaxf(fminf(tn, re), T.t);
-    if(t1 > T.t) {
-      const float k = gas_k(S, p.q, T.prop, l);
-      const uint32_t z3[3] = {0, 0, 0};
-      if(voxel_filter<V>(p, S, T.t, t1, k, k, false, z3, z3)) { trace_finish(p, true); return; }
-    }
-    if(tn >= re) { ++T.region; region_enter(T, S); return; }
-    T.t = t1;
-    const int ln = l + (T.d.z > 0.f ? 1 : -1);
-    if(ln < 0 || ln >= (int)S.nlayers) { ++T.region; region_enter(T, S); return; }
-    T.layer = ln;
-    return;
-  }
-  /* cloud voxel: descend to the leaf holding the current cell, from the
-   * deepest cached ancestor that also holds it */
-  const uint4* nodes = S.nodes + T.base;
-  uint32_t L, base;
+  uint32_t L = 0;
   uint4 v;
-  bool leaf_root = false;
-  bool found = false;
-  if(S.maj_grid) {
-    /* the leaf's majorants and level from the cell: two independent loads,
-     * no node read */
-    const uint64_t gi = (uint64_t)T.grank * S.ncell
-                      + ((uint64_t)T.c[2] * S.def[1] + T.c[1]) * S.def[0] + T.c[0];
-    const float2 mm = __ldg(S.maj_grid + gi);
-    L = __ldg(S.lvl_grid + gi);
-    p.c_grid += 9;
-    v.x = __float_as_uint(mm.x);
-    v.y = __float_as_uint(mm.y);
-    found = true;
-  } else if(T.start == 1) {
-    base = T.p_base; L = T.p_level;
-  } else if(S.leaf_grid) {
-    /* the leaf from the cell's grid entry: two dependent loads whatever the
-     * depth; its parent's child block is cached for the next steps */
-    const uint64_t cell = ((uint64_t)T.c[2] * S.def[1] + T.c[1]) * S.def[0] + T.c[0];
-    const uint32_t e = __ldg(S.leaf_grid + (uint64_t)T.grank * S.ncell + cell);
-    const uint32_t n = e >> 5;
-    L = e & 31u;
-    v = __ldg(nodes + n);
-    ++p.c_node;
-    p.c_grid += 4;
-    found = true;
-    if(L < S.depth) {
-      const uint32_t oct = ((T.c[0] >> L) & 1u) | (((T.c[1] >> L) & 1u) << 1) | (((T.c[2] >> L) & 1u) << 2);
-      T.p_base = n - oct;
-      T.p_level = (uint8_t)(L + 1);
-    } else {
-      T.p_level = 0xFF; /* the root is the leaf: no ancestor */
-    }
-    T.g_level = 0xFF;
-  } else if(T.start == 2) {
-    base = T.g_base; L = T.g_level;
-    T.p_base = base; T.p_level = (uint8_t)L; T.g_level = 0xFF;
-  } else {
-    v = __ldg(nodes);
-    ++p.c_node;
-    L = S.depth;
-    base = v.z;
-    T.p_base = base; T.p_level = (uint8_t)L; T.g_level = 0xFF;
-    leaf_root = v.z == HG_LEAF;
-  }
-  if(!leaf_root && !found) {
-    for(;;) {
-      --L;
-      const uint32_t oct = ((T.c[0] >> L) & 1u) | (((T.c[1] >> L) & 1u) << 1) | (((T.c[2] >> L) & 1u) << 2);
-      v = __ldg(nodes + base + oct);
-      ++p.c_node;
-      if(v.z == HG_LEAF) break;
-      T.g_base = T.p_base; T.g_level = T.p_level;
-      T.p_base = v.z; T.p_level = (uint8_t)L;
-      base = v.z;
-    }
-  } else if(leaf_root) {
-    T.p_level = 0xFF; /* the root is the leaf: no ancestor */
-  }
-  uint32_t lo[3], hi[3];
+  Voxel vx;
+  uint32_t* lo = vx.lo;
+  uint32_t* hi = vx.hi;
   float texit = FLT_MAX;
   int axis = -1;
-#pragma unroll
-  for(int a = 0; a < 3; ++a) {
-    lo[a] = (T.c[a] >> L) << L;
-    hi[a] = min(lo[a] + (1u << L), S.def[a]);
-    const float off = a < 2 ? (float)(T.tile[a] * (int)S.def[a]) : 0.f;
-    const float da = comp(T.d, a);
-    float ta;
-    if(da > 0.f) ta = (S.lower[a] + (off + (float)hi[a]) * S.cell[a] - comp(T.o, a)) * comp(T.inv, a);
-    else if(da < 0.f) ta = (S.lower[a] + (off + (float)lo[a]) * S.cell[a] - comp(T.o, a)) * comp(T.inv, a);
-    else continue;
-    if(ta < texit) { texit = ta; axis = a; }
+  if(!cloud) { /* a horizontal ray stays in its gas layer to the region's end */
+    v.x = v.y = __float_as_uint(gas_k(S, p.q, T.prop, T.layer));
+  } else {
+    /* cloud voxel: descend to the leaf holding the current cell, from the
+     * deepest cached ancestor that also holds it */
+    const uint4* nodes = S.nodes + T.base;
+    uint32_t base;
+    bool leaf_root = false;
+    bool found = false;
+    if(S.maj_grid) {
+      /* the leaf's majorants and level from the cell: two independent loads,
+       * no node read */
+      const uint64_t gi = (uint64_t)T.grank * S.ncell + (uint64_t)T.c[0] * S.gstride[0]
+                        + (uint64_t)T.c[1] * S.gstride[1] + (uint64_t)T.c[2] * S.gstride[2];
+      const float2 mm = __ldg(S.maj_grid + gi);
+      L = __ldg(S.lvl_grid + gi);
+      p.c_grid += 9;
+      v.x = __float_as_uint(mm.x);
+      v.y = __float_as_uint(S.maj_flag ? fabsf(mm.y) : mm.y);
+      found = true;
+    } else if(T.start == 1) {
+      base = T.p_base; L = T.p_level;
+    } else if(S.leaf_grid) {
+      /* the leaf from the cell's grid entry: two dependent loads whatever the
+       * depth; its parent's child block is cached for the next steps */
+      const uint64_t cell = ((uint64_t)T.c[2] * S.def[1] + T.c[1]) * S.def[0] + T.c[0];
+      const uint32_t e = __ldg(S.leaf_grid + (uint64_t)T.grank * S.ncell + cell);
+      const uint32_t n = e >> 5;
+      L = e & 31u;
+      v = __ldg(nodes + n);
+      ++p.c_node;
+      p.c_grid += 4;
+      found = true;
+      if(L < S.depth) {
+        const uint32_t oct = ((T.c[0] >> L) & 1u) | (((T.c[1] >> L) & 1u) << 1) | (((T.c[2] >> L) & 1u) << 2);
+        T.p_base = n - oct;
+        T.p_level = (uint8_t)(L + 1);
+      } else {
+        T.p_level = 0xFF; /* the root is the leaf: no ancestor */
+      }
+      T.g_level = 0xFF;
+    } else if(T.start == 2) {
+      base = T.g_base; L = T.g_level;
+      T.p_base = base; T.p_level = (uint8_t)L; T.g_level = 0xFF;
+    } else {
+      v = __ldg(nodes);
+      ++p.c_node;
+      L = S.depth;
+      base = v.z;
+      T.p_base = base; T.p_level = (uint8_t)L; T.g_level = 0xFF;
+      leaf_root = v.z == HG_LEAF;
+    }
+    if(!leaf_root && !found) {
+      for(;;) {
+        --L;
+        const uint32_t oct = ((T.c[0] >> L) & 1u) | (((T.c[1] >> L) & 1u) << 1) | (((T.c[2] >> L) & 1u) << 2);
+        v = __ldg(nodes + base + oct);
+        ++p.c_node;
+        if(v.z == HG_LEAF) break;
+        T.g_base = T.p_base; T.g_level = T.p_level;
+        T.p_base = v.z; T.p_level = (uint8_t)L;
+        base = v.z;
+      }
+    } else if(leaf_root) {
+      T.p_level = 0xFF; /* the root is the leaf: no ancestor */
+    }
+  #pragma unroll
+    for(int a = 0; a < 3; ++a) {
+      lo[a] = (T.c[a] >> L) << L;
+      hi[a] = min(lo[a] + (1u << L), S.def[a]);
+      const float off = a < 2 ? (float)(T.tile[a] * (int)S.def[a]) : 0.f;
+      const float da = comp(T.d, a);
+      float ta;
+      if(da > 0.f) ta = (S.lower[a] + (off + (float)hi[a]) * S.cell[a] - comp(T.o, a)) * comp(T.inv, a);
+      else if(da < 0.f) ta = (S.lower[a] + (off + (float)lo[a]) * S.cell[a] - comp(T.o, a)) * comp(T.inv, a);
+      else continue;
+      if(ta < texit) { texit = ta; axis = a; }
+    }
   }
   const float t1 = fmaxf(fminf(texit, re), T.t);
   if(t1 > T.t) {
-    if(voxel_filter<V>(p, S, T.t, t1, __uint_as_float(v.x), __uint_as_float(v.y), true, lo, hi)) {
+    if(voxel_filter<V>(p, S, T.t, t1, __uint_as_float(v.x), __uint_as_float(v.y), cloud, vx)) {
       trace_finish(p, true);
       return;
     }
   }
-  if(texit >= re || axis < 0) { ++T.region; region_enter(T, S); return; }
+  if(texit >= re || axis < 0) { region_leave(p); return; }
   /* next cell: exit face on `axis', the exit point's cell on the others */
   const float3 pe = madd3(T.o, T.d, texit);
   uint32_t nc3[3];
@@ -949,6 +1003,8 @@ trace_step(Path& p, const DScene& S)
           leave = true;
         }
       }
+    } else if(L == 0) { /* a leaf of one cell */
+      nc = (int)T.c[a];
     } else {
       int g = __float2int_rd((comp(pe, a) - S.lower[a]) * S.inv_cell[a]);
       if(a < 2) g -= T.tile[a] * (int)S.def[a];
@@ -956,8 +1012,8 @@ trace_step(Path& p, const DScene& S)
     }
     nc3[a] = (uint32_t)nc;
   }
-  if(leave) { ++T.region; region_enter(T, S); return; }
-  { /* deepest cached ancestor whose cube also holds the next cell */
+  if(leave) { region_leave(p); return; }
+  if(!S.maj_grid) { /* deepest cached ancestor whose cube also holds the next cell */
     const uint32_t diff = (T.c[0] ^ nc3[0]) | (T.c[1] ^ nc3[1]) | (T.c[2] ^ nc3[2]);
     if(T.p_level < 32 && (diff >> T.p_level) == 0) T.start = 1;
     else if(T.g_level < 32 && (diff >> T.g_level) == 0) T.start = 2;
@@ -967,6 +1023,15 @@ trace_step(Path& p, const DScene& S)
   T.c[1] = nc3[1];
   T.c[2] = nc3[2];
   T.t = texit;
+}
+
+/* One voxel of the current trace */
+template <unsigned V>
+__device__ __forceinline__ void
+trace_step(PathTrace& p, const DScene& S)
+{
+  trace_enter(p.tr, S);
+  trace_voxel<V>(p, S);
 }
 
 /*******************************************************************************
@@ -1036,10 +1101,9 @@ __device__ __noinline__ GenOut
 gen_sample(const DScene& S, const DRequest& R, uint32_t pix, uint32_t ireal)
 {
   GenOut g;
-  Path p; /* scratch holder so that the shared helpers below keep their form */
+  struct { Rng rng; uint32_t chan; float3 org, rdir; } p;
   const uint32_t px = pix % R.width, py = pix / R.width;
   p.rng.init(pix, R.seed, ireal, 0u);
-  p.flags = 0;
   p.chan = R.mode == HG_IMAGE_CIE ? (uint8_t)(ireal / R.spp) : 0;
   g.chan = p.chan;
   g.cosN = 0.f;
@@ -1137,27 +1201,27 @@ gen_sample(const DScene& S, const DRequest& R, uint32_t pix, uint32_t ireal)
  * wavelength, band and quadrature point (draw_map.c:51-107, 134-177,
  * 233-263, 348-384). */
 __device__ __forceinline__ void
-path_generate(Path& p, const DScene& S, const DRequest& R)
+path_generate(PathTrace& p, PathEvent& e, const DScene& S, const DRequest& R)
 {
   const GenOut g = gen_sample(S, R, p.pix, p.ireal);
-  p.w = 0.0;
-  p.wdirect = 0.0;
+  e.w = 0.0;
+  e.wdirect = 0.0;
   p.c_seg = p.c_node = p.c_tc = p.c_grid = 0;
   p.t0 = gtimer();
   p.rng = g.rng;
   p.chan = (uint8_t)g.chan;
   p.flags = g.flags;
-  p.org = g.org;
-  p.rdir = g.rdir;
+  e.org = g.org;
+  e.rdir = g.rdir;
   if(g.flags & PF_REJECTED) { p.state = ST_DONE; return; }
-  p.wlen = (float)g.wlen;
-  p.wlen_d = g.wlen;
+  e.wlen = (float)g.wlen;
+  e.wlen_d = g.wlen;
   p.band = g.band;
   p.q = g.q;
-  p.inv_pdf = g.inv_pdf;
-  p.cosN = g.cosN;
-  p.pos = g.org;
-  p.dir = g.dir;
+  e.inv_pdf = g.inv_pdf;
+  e.cosN = g.cosN;
+  e.pos = g.org;
+  e.dir = g.dir;
   p.state = ST_RAD_BEGIN;
 }
 
@@ -1187,6 +1251,8 @@ sw_scatter(const DScene& S, Rng rng, float3 dir, float g, uint32_t flags, float 
   int brdf_specular = 0;
   o.refl = refl;
   o.sdir = mk3(0.f, 0.f, 0.f);
+  float3 axis = dir; /* diffuse directions: around this axis */
+  float mu, az;
   if(surface) {
     const SurfProps sp = surface_props<V>(S, rng, dir, gprim, gN, wlen_nm);
     N = sp.N;
@@ -1194,11 +1260,13 @@ sw_scatter(const DScene& S, Rng rng, float3 dir, float g, uint32_t flags, float 
     if(dot3(N, wo) < 0.f) N = neg3(N);
     o.refl = sp.refl;
     if(sp.specular) {
-      o.dnext = nrm3(add3(mul3(N, 2.f * dot3(N, wo)), neg3(wo)));
+      o.dnext = reflect3(N, wo);
       specular = true;
     } else {
       const float u1 = rng.uf(), u2 = rng.uf();
-      o.dnext = around(N, sqrtf(1.f - u2), u1);
+      axis = N;
+      mu = sqrtf(1.f - u2);
+      az = u1;
     }
     flags &= ~PF_RAYLEIGH;
   } else {
@@ -1208,8 +1276,10 @@ sw_scatter(const DScene& S, Rng rng, float3 dir, float g, uint32_t flags, float 
     const bool ray = (double)rng.uf() < ks_gas / ks;
     if(ray) flags |= PF_RAYLEIGH; else flags &= ~PF_RAYLEIGH;
     const float u1 = rng.uf(), u2 = rng.uf();
-    o.dnext = around(dir, ray ? rayleigh_mu(u1) : hg_mu(g, u1), u2);
+    mu = ray ? rayleigh_mu(u1) : hg_mu(g, u1);
+    az = u2;
   }
+  if(!specular) o.dnext = around(axis, mu, az);
   if(specular) flags |= PF_SPECULAR; else flags &= ~PF_SPECULAR;
   if(surface && specular) {
     if(!in_solar_cone(S, o.dnext)) o.R = 0.f;
@@ -1233,7 +1303,7 @@ sw_scatter(const DScene& S, Rng rng, float3 dir, float g, uint32_t flags, float 
 
 /* A path of a kind the kernel variant leaves out: a failed realisation */
 __device__ __forceinline__ void
-path_variant_miss(Path& p)
+path_variant_miss(PathTrace& p)
 {
   p.flags |= PF_FAILED;
   p.state = ST_RAD_END;
@@ -1257,37 +1327,49 @@ lw_plane_ground(const DScene& S)
  * from the collision site, the head of the walk (..._lw.c:184-205) -- the
  * steps ST_LW_END and ST_LW_WALK take there.  It reads and writes the trace
  * part of the path only (the plane's hit record, set at the walk's first
- * ground query, stays the same) and returns the walk's new position and
- * direction, which the wavefront's trace stage stores into p.pos / p.dir:
- * the stage runs it without an event-stage visit.  The caller checks that
+ * ground query, stays the same); the origin and direction of the free path it
+ * asks for are the walk's new position and direction, which the wavefront's
+ * trace stage stores into p.pos / p.dir: the stage runs it without an
+ * event-stage visit.  The caller checks that
  * the bounce limit is not reached. */
 __device__ __forceinline__ void
-lw_scatter_plane(Path& p, const DScene& S, float3& pos, float3& dir)
+lw_scatter_plane(PathTrace& p, const DScene& S, TraceArgs& q)
 {
-  pos = madd3(p.tr.o, p.tr.d, p.tr.tcur);
   const float g = __ldg(S.optics + p.band).w;
   const float u1 = p.rng.uf(), u2 = p.rng.uf();
-  dir = around(p.tr.d, hg_mu(g, u1), u2);
+  q.kind = TK_LW;
+  q.prop = HG_KEXT;
+  q.ret = ST_LW_END;
+  q.o = madd3(p.tr.o, p.tr.d, p.tr.tcur);
+  q.d = around(p.tr.d, hg_mu(g, u1), u2);
   p.flags &= ~PF_PREV_GROUND;
   ++p.bounces;
-  p.gdist = ground_trace(S, pos, dir, 0.f, FLT_MAX, false);
-  p.tr.Ts = p.rng.exp1();
-  trace_begin(p, S, TK_LW, HG_KEXT, pos, dir, 0.f, p.gdist >= 0.f ? p.gdist : FLT_MAX, ST_LW_END);
+  p.gdist = ground_trace(S, q.o, q.d, 0.f, FLT_MAX, false);
+  q.t1 = p.gdist >= 0.f ? p.gdist : FLT_MAX;
 }
 
 template <unsigned V>
 __device__ __forceinline__ void
-path_event(Path& p, const DScene& S, const DRequest& R)
+path_event(PathTrace& p, PathEvent& e, const DScene& S, const DRequest& R)
 {
-  for(;;) {
+  /* transmissivity of the trace that just ended, where the state wants one:
+   * one exponential in the kernel, as the trace is begun in one place */
+  double Tr = 0.0;
+  if(V & HV_SW) {
+    if(p.state == ST_SW_ABS_END || p.state == ST_SW_NEE_END || p.state == ST_SW_DIRECT_END)
+      Tr = p.tr.hit ? 0.0 : (p.tr.Tmin != 0.0 ? exp(-p.tr.Tmin) : 1.0);
+  }
+  TraceArgs q;
+  bool begin = false;
+  while(!begin) {
     switch(p.state) {
-      case ST_GEN: path_generate(p, S, R); break;
+      case ST_GEN: path_generate(p, e, S, R); break;
 
       case ST_RAD_BEGIN: {
-        p.g = __ldg(S.optics + p.band).w;
+        e.g = __ldg(S.optics + p.band).w;
         p.flags &= ~(PF_PREV_GROUND | PF_TRACED);
-        p.w = 0.0;
-        p.ksi = 1.f;
+        e.w = 0.0;
+        e.ksi = 1.f;
         p.bounces = 0;
         if(p.flags & PF_LW) {
           if(V & HV_LW) p.state = ST_LW_WALK;
@@ -1296,18 +1378,18 @@ path_event(Path& p, const DScene& S, const DRequest& R)
         }
         if constexpr(!(V & HV_SW)) { path_variant_miss(p); break; }
         else {
-        p.L_sun = planck_mono(p.wlen_d * 1e-9, S.sun_T);
-        if((p.flags & PF_DIRECT) && ((p.flags & PF_IN_CONE) || in_solar_cone(S, p.dir))) {
+        e.L_sun = planck_mono(e.wlen_d * 1e-9, S.sun_T);
+        p.state = ST_SW_DIRECT_END;
+        if((p.flags & PF_DIRECT) && ((p.flags & PF_IN_CONE) || in_solar_cone(S, e.dir))) {
           uint32_t hp;
           bool he;
           float3 hn;
-          if(ground_query<V>(S, p.pos, p.dir, FLT_MAX, false, 0u, false, &hp, &he, &hn) < 0.f) {
+          if(ground_query<V>(S, e.pos, e.dir, FLT_MAX, false, 0u, false, &hp, &he, &hn) < 0.f) {
             p.flags |= PF_TRACED;
-            trace_begin(p, S, TK_TRANS, HG_KEXT, p.pos, p.dir, 0.f, FLT_MAX, ST_SW_DIRECT_END);
-            return;
+            q = TraceArgs{TK_TRANS, HG_KEXT, ST_SW_DIRECT_END, e.pos, e.dir, FLT_MAX};
+            begin = true;
           }
         }
-        p.state = ST_SW_DIRECT_END;
         break;
         }
       }
@@ -1315,63 +1397,64 @@ path_event(Path& p, const DScene& S, const DRequest& R)
       case ST_SW_DIRECT_END:
         if constexpr(!(V & HV_SW)) { path_variant_miss(p); break; }
         else {
-          if(p.flags & PF_TRACED) {
-            const double Tr = p.tr.hit ? 0.0 : (p.tr.Tmin != 0.0 ? exp(-p.tr.Tmin) : 1.0);
-            p.w = p.L_sun * Tr;
-          }
+          if(p.flags & PF_TRACED) e.w = e.L_sun * Tr;
           p.state = (p.flags & PF_DIFFUSE) ? ST_SW_WALK : ST_RAD_END;
         }
         break;
 
-      case ST_SW_WALK: if constexpr(!(V & HV_SW)) { path_variant_miss(p); break; } else {
+      case ST_SW_WALK:
+      case ST_LW_WALK: { /* the next free path */
+        const bool lw = (V & HV_LW) && (!(V & HV_SW) || p.state == ST_LW_WALK);
+        if(p.state == ST_LW_WALK ? !(V & HV_LW) : !(V & HV_SW)) { path_variant_miss(p); break; }
         if(++p.bounces > HG_MAX_BOUNCES) { p.flags |= PF_FAILED; p.state = ST_RAD_END; break; }
-        {
-          bool e;
-          p.gdist = ground_query<V>(S, p.pos, p.dir, FLT_MAX, (p.flags & PF_PREV_GROUND) != 0,
-                                 p.prev_prim, p.prev_edge != 0, &p.gprim, &e, &p.gN);
-          p.gedge = e;
-        }
-        p.tr.Ts = p.rng.exp1();
-        trace_begin(p, S, TK_SCATTER, HG_KS, p.pos, p.dir, 0.f,
-                    p.gdist >= 0.f ? p.gdist : FLT_MAX, ST_SW_SCAT_END);
-        return;
+        bool edge;
+        p.gdist = ground_query<V>(S, e.pos, e.dir, FLT_MAX, (p.flags & PF_PREV_GROUND) != 0,
+                                  e.prev_prim, e.prev_edge != 0, &e.gprim, &edge, &e.gN);
+        e.gedge = edge;
+        q = TraceArgs{lw ? TK_LW : TK_SCATTER, lw ? HG_KEXT : HG_KS,
+                      (uint8_t)(lw ? ST_LW_END : ST_SW_SCAT_END), e.pos, e.dir,
+                      p.gdist >= 0.f ? p.gdist : FLT_MAX};
+        begin = true;
+        break;
       }
 
       case ST_SW_SCAT_END: if constexpr(!(V & HV_SW)) { path_variant_miss(p); break; } else {
-        if(p.tr.hit) { p.pnext = sw_scat_volume(p, S); return; } /* the trace origin is p.pos */
+        if(p.tr.hit) { e.pnext = sw_scat_volume(p, q); begin = true; break; } /* the trace origin is e.pos */
         if(p.gdist < 0.f) { p.state = ST_RAD_END; break; }
         /* the ground: scattering at the surface */
         const float tdst = p.gdist;
-        p.pnext = madd3(p.pos, p.dir, tdst);
+        e.pnext = madd3(e.pos, e.dir, tdst);
         p.flags |= PF_SURFACE | PF_PREV_GROUND;
-        p.prev_prim = p.gprim;
-        p.prev_edge = p.gedge;
-        trace_begin(p, S, TK_TRANS, HG_KA, p.pos, p.dir, 0.f, tdst, ST_SW_ABS_END);
-        return;
+        e.prev_prim = e.gprim;
+        e.prev_edge = e.gedge;
+        q = TraceArgs{TK_TRANS, HG_KA, ST_SW_ABS_END, e.pos, e.dir, tdst};
+        begin = true;
+        break;
       }
 
       case ST_SW_ABS_END: if constexpr(!(V & HV_SW)) { path_variant_miss(p); break; } else {
-        p.tr_abs = p.tr.hit ? 0.f : (float)(p.tr.Tmin != 0.0 ? exp(-p.tr.Tmin) : 1.0);
-        if(p.tr_abs <= 0.f) { p.state = ST_RAD_END; break; }
+        e.tr_abs = (float)Tr;
+        if(e.tr_abs <= 0.f) { p.state = ST_RAD_END; break; }
         /* the collision site of the free path: the absorption trace keeps it */
-        const ScatOut so = sw_scatter<V>(S, p.rng, p.dir, p.g, p.flags, p.refl, p.tr.site_cell,
-                                      p.tr.site_layer, p.band, p.q, p.gprim, p.gN, p.wlen_d);
+        const ScatOut so = sw_scatter<V>(S, p.rng, e.dir, e.g, p.flags, e.refl, p.tr.site_cell,
+                                      p.tr.site_layer, p.band, p.q, e.gprim, e.gN, e.wlen_d);
         p.rng = so.rng;
         p.flags = so.flags;
-        p.dnext = so.dnext;
-        p.sdir = so.sdir;
-        p.R = so.R;
-        p.refl = so.refl;
-        p.sun_ipdf = so.sun_ipdf;
+        e.dnext = so.dnext;
+        e.sdir = so.sdir;
+        e.R = so.R;
+        e.refl = so.refl;
+        e.sun_ipdf = so.sun_ipdf;
         uint32_t hp;
         bool he;
         float3 hn;
-        if(p.R > 0.f
-        && ground_query<V>(S, p.pnext, p.sdir, FLT_MAX, (p.flags & PF_PREV_GROUND) != 0, p.prev_prim,
-                        p.prev_edge != 0, &hp, &he, &hn) < 0.f) {
+        if(e.R > 0.f
+        && ground_query<V>(S, e.pnext, e.sdir, FLT_MAX, (p.flags & PF_PREV_GROUND) != 0, e.prev_prim,
+                        e.prev_edge != 0, &hp, &he, &hn) < 0.f) {
           p.flags |= PF_TRACED;
-          trace_begin(p, S, TK_TRANS, HG_KEXT, p.pnext, p.sdir, 0.f, FLT_MAX, ST_SW_NEE_END);
-          return;
+          q = TraceArgs{TK_TRANS, HG_KEXT, ST_SW_NEE_END, e.pnext, e.sdir, FLT_MAX};
+          begin = true;
+          break;
         }
         p.flags &= ~PF_TRACED;
         p.state = ST_SW_NEE_END;
@@ -1379,74 +1462,70 @@ path_event(Path& p, const DScene& S, const DRequest& R)
       }
 
       case ST_SW_NEE_END: if constexpr(!(V & HV_SW)) { path_variant_miss(p); break; } else {
-        double Tr = 0.0;
-        if(p.flags & PF_TRACED) Tr = p.tr.hit ? 0.0 : (p.tr.Tmin != 0.0 ? exp(-p.tr.Tmin) : 1.0);
+        const double Ts = (p.flags & PF_TRACED) ? Tr : 0.0;
         p.flags &= ~PF_TRACED;
-        p.ksi *= p.tr_abs;
-        p.w += (double)p.ksi * p.L_sun * Tr * (double)p.R * (double)p.sun_ipdf;
-        if((p.flags & PF_SURFACE) && p.rng.uf() >= p.refl) { p.state = ST_RAD_END; break; }
-        p.pos = p.pnext;
-        p.dir = p.dnext;
+        e.ksi *= e.tr_abs;
+        e.w += (double)e.ksi * e.L_sun * Ts * (double)e.R * (double)e.sun_ipdf;
+        if((p.flags & PF_SURFACE) && p.rng.uf() >= e.refl) { p.state = ST_RAD_END; break; }
+        e.pos = e.pnext;
+        e.dir = e.dnext;
         p.state = ST_SW_WALK;
         break;
-      }
-
-      case ST_LW_WALK: if constexpr(!(V & HV_LW)) { path_variant_miss(p); break; } else {
-        if(++p.bounces > HG_MAX_BOUNCES) { p.flags |= PF_FAILED; p.state = ST_RAD_END; break; }
-        {
-          bool e;
-          p.gdist = ground_query<V>(S, p.pos, p.dir, FLT_MAX, (p.flags & PF_PREV_GROUND) != 0,
-                                 p.prev_prim, p.prev_edge != 0, &p.gprim, &e, &p.gN);
-          p.gedge = e;
-        }
-        p.tr.Ts = p.rng.exp1();
-        trace_begin(p, S, TK_LW, HG_KEXT, p.pos, p.dir, 0.f,
-                    p.gdist >= 0.f ? p.gdist : FLT_MAX, ST_LW_END);
-        return;
       }
 
       case ST_LW_END: if constexpr(!(V & HV_LW)) { path_variant_miss(p); break; } else {
         /* the free path just traced started at p.tr.o along p.tr.d (the
          * walk's position and direction, which the trace stage may have
-         * moved past p.pos / p.dir) */
+         * moved past e.pos / e.dir) */
         const bool svx = p.tr.hit != 0;
-        const double wlen_m = p.wlen_d * 1e-9;
-        if(p.gdist < 0.f && !svx) { p.w = 0.0; p.state = ST_RAD_END; break; }
+        if(p.gdist < 0.f && !svx) { e.w = 0.0; p.state = ST_RAD_END; break; }
         const float tdst = svx ? p.tr.tcur : p.gdist;
-        p.pnext = madd3(p.pos, p.dir, tdst);
+        e.pnext = madd3(e.pos, e.dir, tdst);
+        double emit = -1.0; /* temperature of the emission that ends the walk */
+        bool ends = false, specular = false;
+        float3 axis = e.dir;
+        float mu = 0.f, az = 0.f;
         if(svx && p.tr.event == 0) {
-          const int l = p.tr.site_layer >= 0 ? p.tr.site_layer : layer_of(S, p.pnext.z);
-          p.w = planck_mono(wlen_m, (double)__ldg(S.layer_T + l));
+          const int l = p.tr.site_layer >= 0 ? p.tr.site_layer : layer_of(S, e.pnext.z);
+          emit = (double)__ldg(S.layer_T + l);
+          ends = true;
+        } else if(svx) {
+          const float u1 = p.rng.uf(), u2 = p.rng.uf();
+          mu = hg_mu(e.g, u1);
+          az = u2;
+          p.flags &= ~PF_PREV_GROUND;
+        } else {
+          const SurfProps sp = surface_props<V>(S, p.rng, e.dir, e.gprim, e.gN, e.wlen_d);
+          float3 N = sp.N;
+          const float3 wo = neg3(e.dir);
+          if(dot3(N, wo) < 0.f) N = neg3(N);
+          specular = sp.specular != 0;
+          if(specular) {
+            e.dnext = reflect3(N, wo);
+          } else {
+            const float u1 = p.rng.uf(), u2 = p.rng.uf();
+            axis = N;
+            mu = sqrtf(1.f - u2);
+            az = u1;
+          }
+          if(p.rng.uf() >= sp.refl) {
+            emit = (double)sp.T;
+            ends = true;
+          } else {
+            p.flags |= PF_PREV_GROUND;
+            e.prev_prim = e.gprim;
+            e.prev_edge = e.gedge;
+          }
+        }
+        if(ends) {
+          /* a surface at 0 K emits nothing */
+          e.w = svx || emit > 0 ? planck_mono(e.wlen_d * 1e-9, emit) : 0.0;
           p.state = ST_RAD_END;
           break;
         }
-        if(svx) {
-          const float u1 = p.rng.uf(), u2 = p.rng.uf();
-          p.dnext = around(p.dir, hg_mu(p.g, u1), u2);
-          p.flags &= ~PF_PREV_GROUND;
-        } else {
-          const SurfProps sp = surface_props<V>(S, p.rng, p.dir, p.gprim, p.gN, p.wlen_d);
-          float3 N = sp.N;
-          const float3 wo = neg3(p.dir);
-          if(dot3(N, wo) < 0.f) N = neg3(N);
-          if(sp.specular) {
-            p.dnext = nrm3(add3(mul3(N, 2.f * dot3(N, wo)), neg3(wo)));
-          } else {
-            const float u1 = p.rng.uf(), u2 = p.rng.uf();
-            p.dnext = around(N, sqrtf(1.f - u2), u1);
-          }
-          if(p.rng.uf() >= sp.refl) {
-            const double T = (double)sp.T;
-            p.w = T > 0 ? planck_mono(wlen_m, T) : 0.0;
-            p.state = ST_RAD_END;
-            break;
-          }
-          p.flags |= PF_PREV_GROUND;
-          p.prev_prim = p.gprim;
-          p.prev_edge = p.gedge;
-        }
-        p.pos = p.pnext;
-        p.dir = p.dnext;
+        if(!specular) e.dnext = around(axis, mu, az);
+        e.pos = e.pnext;
+        e.dir = e.dnext;
         p.state = ST_LW_WALK;
         break;
       }
@@ -1454,16 +1533,19 @@ path_event(Path& p, const DScene& S, const DRequest& R)
       case ST_RAD_END:
         if((V & HV_SW) && R.mode == HG_FLUX_SW) {
           if(!(p.flags & PF_STAGE2)) {
-            p.wdirect = p.w;
+            e.wdirect = e.w;
             p.flags = (p.flags & ~(PF_DIRECT | PF_IN_CONE)) | PF_STAGE2 | PF_DIFFUSE;
-            p.pos = p.org;
-            p.dir = p.rdir;
+            e.pos = e.org;
+            e.dir = e.rdir;
             p.state = ST_RAD_BEGIN;
             break;
           }
-          p.weight = ((double)p.cosN * S.sun_solid_angle * p.wdirect + HG_PI_D * p.w) * p.inv_pdf;
+          { /* cos x solid angle x direct + pi x diffuse */
+            const double cs = __dmul_rn((double)e.cosN, S.sun_solid_angle);
+            e.weight = fma(cs, e.wdirect, __dmul_rn(HG_PI_D, e.w)) * e.inv_pdf;
+          }
         } else {
-          p.weight = p.w * p.inv_pdf;
+          e.weight = e.w * e.inv_pdf;
         }
         p.state = ST_DONE;
         return;
@@ -1472,6 +1554,7 @@ path_event(Path& p, const DScene& S, const DRequest& R)
         return;
     }
   }
+  trace_begin(p, S, q);
 }
 
 }  // namespace

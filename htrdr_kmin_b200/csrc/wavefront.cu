@@ -26,6 +26,7 @@
  * kernel).  Every path is bounded in bounces and voxel steps, so the loop
  * ends. */
 #include "engine.cuh"
+#include "walk.cuh"
 
 #include <algorithm>
 #include <map>
@@ -37,20 +38,22 @@ namespace hg {
 namespace {
 
 constexpr uint32_t kPathV4 = (uint32_t)((sizeof(Path) + 15) / 16);
-constexpr uint32_t kTraceV4 = (uint32_t)((offsetof(Path, org) + 15) / 16);
-static_assert(kTraceV4 <= kPathV4, "trace part inside the path");
+constexpr uint32_t kTraceV4 = (uint32_t)(sizeof(PathTrace) / 16);
+static_assert(sizeof(PathTrace) % 16 == 0, "the trace part is whole vectors");
+/* Offset of a field of the event part in a stored path */
+#define HG_EVENT_AT(f) (sizeof(PathTrace) + offsetof(PathEvent, f))
 /* The vector holding the collision site of a SW free path (pnext), which the
  * trace stage writes when it runs the absorption trace itself.  Its last
  * word is dnext.x, dead from there until ST_SW_ABS_END sets dnext. */
-constexpr uint32_t kPnextV4 = (uint32_t)(offsetof(Path, pnext) / 16);
-static_assert(offsetof(Path, pnext) % 16 == 0 && offsetof(Path, dnext) == offsetof(Path, pnext) + 12,
+constexpr uint32_t kPnextV4 = (uint32_t)(HG_EVENT_AT(pnext) / 16);
+static_assert(HG_EVENT_AT(pnext) % 16 == 0 && HG_EVENT_AT(dnext) == HG_EVENT_AT(pnext) + 12,
               "pnext and dnext.x fill one 16-byte vector");
 /* The vectors of the walk's position and direction, which the trace stage
  * writes when it runs a LW scattering itself: pos.x, pos.y end the first,
  * pos.z and dir fill the second */
-constexpr uint32_t kPosV4 = (uint32_t)(offsetof(Path, pos) / 16);
-static_assert(offsetof(Path, pos) % 16 == 8 && offsetof(Path, dir) == offsetof(Path, pos) + 12
-              && offsetof(Path, dir) + 12 == (kPosV4 + 2) * 16, "pos and dir end two 16-byte vectors");
+constexpr uint32_t kPosV4 = (uint32_t)(HG_EVENT_AT(pos) / 16);
+static_assert(HG_EVENT_AT(pos) % 16 == 8 && HG_EVENT_AT(dir) == HG_EVENT_AT(pos) + 12
+              && HG_EVENT_AT(dir) + 12 == (kPosV4 + 2) * 16, "pos and dir end two 16-byte vectors");
 
 /* Gas-region batching of the trace stage (0: off).  Measured on a B200
  * (Mrealisations/s, off / batch 4 wait 8 / batch 8 wait 16): full-size mix
@@ -123,10 +126,9 @@ store_path(const Path& p, uint4* paths, uint32_t s, uint32_t P)
   for(uint32_t i = 0; i < kPathV4; ++i) paths[vec_at(s, i, P)] = v[i];
 }
 
-/* The trace part and the bytes up to the next 16-byte boundary (stored back
- * unchanged) */
+/* The trace part */
 __device__ __forceinline__ void
-load_trace(Path& p, const uint4* paths, uint32_t s, uint32_t P)
+load_trace(PathTrace& p, const uint4* paths, uint32_t s, uint32_t P)
 {
   uint4 v[kTraceV4];
 #pragma unroll
@@ -135,7 +137,7 @@ load_trace(Path& p, const uint4* paths, uint32_t s, uint32_t P)
 }
 
 __device__ __forceinline__ void
-store_trace(const Path& p, uint4* paths, uint32_t s, uint32_t P)
+store_trace(const PathTrace& p, uint4* paths, uint32_t s, uint32_t P)
 {
   uint4 v[kTraceV4];
   memcpy(v, &p, kTraceV4 * 16);
@@ -143,11 +145,21 @@ store_trace(const Path& p, uint4* paths, uint32_t s, uint32_t P)
   for(uint32_t i = 0; i < kTraceV4; ++i) paths[vec_at(s, i, P)] = v[i];
 }
 
+/* The event part */
+__device__ __forceinline__ void
+load_event(PathEvent& e, const uint4* paths, uint32_t s, uint32_t P)
+{
+  uint4 v[kPathV4 - kTraceV4];
+#pragma unroll
+  for(uint32_t i = kTraceV4; i < kPathV4; ++i) v[i - kTraceV4] = paths[vec_at(s, i, P)];
+  memcpy(&e, v, sizeof(PathEvent));
+}
+
 /* Whether a trace that just ended leads to a transition the trace stage runs
  * itself: the absorption trace after a SW collision in the medium, the next
  * free path after a LW scattering in the medium over a plane ground */
 __device__ __forceinline__ bool
-transition_here(const Path& p, const DScene& S)
+transition_here(const PathTrace& p, const DScene& S)
 {
   if(p.state == ST_SW_SCAT_END) return p.tr.hit != 0;
   return p.state == ST_LW_END && p.tr.hit && p.tr.event == 1 && p.bounces < HG_MAX_BOUNCES
@@ -156,24 +168,30 @@ transition_here(const Path& p, const DScene& S)
 
 /* That transition; the event-part fields it sets are stored into slot s */
 __device__ __forceinline__ void
-transition(Path& p, const DScene& S, uint4* paths, uint32_t s, uint32_t P)
+transition(PathTrace& p, const DScene& S, uint4* paths, uint32_t s, uint32_t P)
 {
+  TraceArgs q;
   if(p.state == ST_SW_SCAT_END) {
-    const float3 pn = sw_scat_volume(p, S);
+    const float3 pn = sw_scat_volume(p, q);
     paths[vec_at(s, kPnextV4, P)] =
       make_uint4(__float_as_uint(pn.x), __float_as_uint(pn.y), __float_as_uint(pn.z), 0u);
   } else {
-    float3 pos, dir;
-    lw_scatter_plane(p, S, pos, dir);
+    lw_scatter_plane(p, S, q);
     uint4* v = paths + vec_at(s, kPosV4, P);
-    ((uint2*)v)[1] = make_uint2(__float_as_uint(pos.x), __float_as_uint(pos.y));
+    ((uint2*)v)[1] = make_uint2(__float_as_uint(q.o.x), __float_as_uint(q.o.y));
     v = paths + vec_at(s, kPosV4 + 1, P);
-    *v = make_uint4(__float_as_uint(pos.z), __float_as_uint(dir.x), __float_as_uint(dir.y),
-                    __float_as_uint(dir.z));
+    *v = make_uint4(__float_as_uint(q.o.z), __float_as_uint(q.d.x), __float_as_uint(q.d.y),
+                    __float_as_uint(q.d.z));
   }
+  trace_begin(p, S, q);
 }
 
 }  // namespace
+
+/* Warps of a block of the finishing kernel */
+#ifndef HG_FINISH_WARPS
+#define HG_FINISH_WARPS 4u
+#endif
 
 /* Control block of a wavefront run (device) */
 struct WTables {
@@ -233,7 +251,7 @@ k_wave_event(WTables W, uint32_t b, int tables_in_smem)
         got = __shfl_sync(0xffffffffu, got, leader);
         if(need) {
           const unsigned rank = __popc(m & ((1u << lane) - 1u));
-          if(rank < got) path_assign(p, T, g0 + rank);
+          if(rank < got) path_assign(p, p.ri, T, g0 + rank);
           else drained = true;
         }
       }
@@ -241,12 +259,12 @@ k_wave_event(WTables W, uint32_t b, int tables_in_smem)
       if(!__any_sync(0xffffffffu, busy)) break;
       if(busy) {
         if(p.state != ST_DONE) {
-          path_event<V>(p, T.scenes[p.si], T.reqs[p.ri]);
+          path_event<V>(p, p, T.scenes[p.si], T.reqs[p.ri]);
           seg += p.c_seg; node += p.c_node; tc += p.c_tc;
           p.c_seg = p.c_node = p.c_tc = 0;
         }
         if(p.state == ST_DONE) {
-          accumulate_b(p, T.reqs[p.ri]);
+          accumulate_b(p, p.weight, T.reqs[p.ri]);
           count_grid(T.cnt, p);
           real += (p.flags & (PF_REJECTED | PF_FAILED)) ? 0 : 1;
           fail += (p.flags & PF_FAILED) ? 1 : 0;
@@ -295,7 +313,7 @@ k_wave_trace(WTables W, uint32_t b, int tables_in_smem)
   const uint32_t* list = b ? W.list0 : W.list1;
   const uint32_t n = ctl->n_live[b ^ 1u];
   const unsigned lane = threadIdx.x & 31u;
-  Path p;
+  PathTrace p;
   p.state = ST_IDLE;
   bool have = false, drained = false;
   uint32_t s = 0, left = 0;
@@ -427,94 +445,156 @@ k_wave_clamp(WTables W)
   if(threadIdx.x == 0 && blockIdx.x == 0) queue_clamp(W.T);
 }
 
-/* The tail of a run: once few paths are live, iterations would cost their
- * launch and one trace's latency each while moving almost no work, so the
- * remaining paths finish in one megakernel launch.  Lanes resume the paths of
- * live list 0 from their slots, then take any realisations left in the work
- * queue; events and traces run in the same thread, events regrouped every
- * `regroup_period' voxel steps as in the persistent engine. */
+/* Registers of the finishing kernel.  255 (8 warps per SM) against 168 (12):
+ * a lone path's bounce takes 5.1 against 5.6 ms (1024 realisations), 88 000
+ * realisations of a flux map 31 against 34 ms; batches of long walks are as
+ * fast with either. */
+#ifndef HG_FINISH_MAXNREG
+#define HG_FINISH_MAXNREG 255
+#endif
+/* A phase's trace goes on until a 1/HG_LAG of the warp's paths is left in it;
+ * these go on when the phase comes round again.  1/4, 1/8 and 1/16 measured
+ * within 5 %, 1/4 first. */
+#ifndef HG_LAG
+#define HG_LAG 4
+#endif
+/* Idle lanes that make a warp take new work: the sensor and spectral sampling
+ * is the longest piece of code, so it waits for a few lanes. */
+#ifndef HG_REFILL
+#define HG_REFILL 8
+#endif
+
+/* The finishing kernel keeps the event part of a lane's path in shared
+ * memory: an odd number of 8-byte words apart, so that a warp's 8-byte
+ * accesses to one field do not conflict */
+static_assert(sizeof(PathEvent) % 16 == 8, "odd number of 8-byte words per slot");
+__host__ __device__ constexpr size_t
+finish_event_bytes()
+{
+  return (sizeof(PathEvent) * 32 * HG_FINISH_WARPS + 15) & ~(size_t)15;
+}
+
+/* The tail of a run, and the whole of one with shortwave requests: a lane per
+ * path, the paths of a warp kept in step.  A shortwave bounce is a free path,
+ * the absorption along it, the scattering and a transmissivity towards the
+ * sun; the loop goes through these phases with all paths of the warp.
+ *
+ * What bounds it: the instruction stream of a bounce (some 4000 instructions,
+ * run once from end to end: half of the stalls of a full SM wait for
+ * instructions) and, in the last third of a run, the latency of the longest
+ * path's bounces (~12 us each).  Hence one copy of every routine in the loop, all
+ * lanes of a warp in one phase, and the traces' frequent part apart
+ * (cell_walk).  Lanes regrouped at every voxel step instead, in whatever state
+ * they are, took 41 us a bounce at the tail of a small image and 72 us at the
+ * tail of a flux map; 47 and 128 ms against 16 and 31 ms for the whole calls. */
 template <unsigned V>
-__global__ void __maxnreg__(HG_PERSIST_MAXNREG)
-k_wave_finish(WTables W, int tables_in_smem)
+__global__ void __maxnreg__(HG_FINISH_MAXNREG)
+k_wave_finish(WTables W, int tables_in_smem, uint32_t cap)
 {
   extern __shared__ __align__(16) unsigned char smem[];
   PTables T = W.T;
-  if(tables_in_smem) tables_to_smem(T, smem);
+  if(tables_in_smem) tables_to_smem(T, smem + finish_event_bytes());
   WCtl* ctl = W.ctl;
   const uint32_t n = ctl->n_live[0];
   const unsigned lane = threadIdx.x & 31u;
-  Path p;
+  PathTrace p;
+  PathEvent& e = ((PathEvent*)smem)[threadIdx.x];
   p.state = ST_IDLE;
   p.flags = 0;
   p.c_seg = p.c_node = p.c_tc = 0;
-  p.ri = p.si = 0;
-  bool list_done = false, drained = false;
-  unsigned long long seg = 0, node = 0, tc = 0, real = 0, fail = 0;
-  const uint32_t period = T.regroup_period > 1 ? T.regroup_period : 1;
+  p.si = 0;
+  bool list_done = n == 0, drained = lane >= cap;
+  /* the block's event counters, in shared memory: ten registers less */
+  __shared__ unsigned long long sums[5];
+  if(threadIdx.x < 5) sums[threadIdx.x] = 0;
+  __syncthreads();
 
-  for(uint32_t it = 0;; ++it) {
-    const unsigned tmask = __ballot_sync(0xffffffffu, p.state == ST_TRACE);
-    if(tmask && (it % period) != 0) {
-      if(p.state == ST_TRACE) trace_step<V>(p, T.scenes[p.si]);
-      continue;
-    }
+  for(;;) {
     /* idle lanes: a saved path of the live list first, then the queue */
-    const bool need_l = p.state == ST_IDLE && !list_done;
-    const unsigned ml = __ballot_sync(0xffffffffu, need_l);
-    if(ml) {
-      const unsigned leader = __ffs(ml) - 1;
-      uint32_t i0 = 0;
-      if(lane == leader) i0 = atomicAdd(&ctl->fetch_finish, (uint32_t)__popc(ml));
-      i0 = __shfl_sync(0xffffffffu, i0, leader);
-      if(need_l) {
-        const uint32_t idx = i0 + __popc(ml & ((1u << lane) - 1u));
-        if(idx < n) {
-          load_path(p, W.paths, W.list0[idx], W.P);
-          p.t0 = gtimer() - p.t0;
-        } else {
-          list_done = true;
+    const unsigned live = __ballot_sync(0xffffffffu, p.state != ST_IDLE);
+    const unsigned idle = __ballot_sync(0xffffffffu, p.state == ST_IDLE && !drained);
+    if(idle && (!live || __popc(idle) >= HG_REFILL)) {
+      const bool need_l = p.state == ST_IDLE && !drained && !list_done;
+      const unsigned ml = __ballot_sync(0xffffffffu, need_l);
+      if(ml) {
+        const unsigned leader = __ffs(ml) - 1;
+        uint32_t i0 = 0;
+        if(lane == leader) i0 = atomicAdd(&ctl->fetch_finish, (uint32_t)__popc(ml));
+        i0 = __shfl_sync(0xffffffffu, i0, leader);
+        if(need_l) {
+          const uint32_t idx = i0 + __popc(ml & ((1u << lane) - 1u));
+          if(idx < n) {
+            load_trace(p, W.paths, W.list0[idx], W.P);
+            load_event(e, W.paths, W.list0[idx], W.P);
+            p.t0 = gtimer() - p.t0;
+          } else {
+            list_done = true;
+          }
+        }
+      }
+      const bool need_q = p.state == ST_IDLE && list_done && !drained;
+      const unsigned mq = __ballot_sync(0xffffffffu, need_q);
+      if(mq) {
+        const unsigned leader = __ffs(mq) - 1;
+        unsigned long long g0 = 0;
+        unsigned got = 0;
+        if(lane == leader) g0 = queue_take(T, (unsigned)__popc(mq), &got);
+        g0 = __shfl_sync(0xffffffffu, g0, leader);
+        got = __shfl_sync(0xffffffffu, got, leader);
+        if(need_q) {
+          const unsigned rank = __popc(mq & ((1u << lane) - 1u));
+          if(rank < got) path_assign(p, e.ri, T, g0 + rank);
+          else drained = true;
         }
       }
     }
-    const bool need_q = p.state == ST_IDLE && list_done && !drained;
-    const unsigned mq = __ballot_sync(0xffffffffu, need_q);
-    if(mq) {
-      const unsigned leader = __ffs(mq) - 1;
-      unsigned long long g0 = 0;
-      unsigned got = 0;
-      if(lane == leader) g0 = queue_take(T, (unsigned)__popc(mq), &got);
-      g0 = __shfl_sync(0xffffffffu, g0, leader);
-      got = __shfl_sync(0xffffffffu, got, leader);
-      if(need_q) {
-        const unsigned rank = __popc(mq & ((1u << lane) - 1u));
-        if(rank < got) path_assign(p, T, g0 + rank);
-        else drained = true;
+    if(!__any_sync(0xffffffffu, p.state != ST_IDLE)) {
+      if(__all_sync(0xffffffffu, drained)) break;
+      continue;
+    }
+    const uint32_t lag = (uint32_t)__popc(__ballot_sync(0xffffffffu, p.state != ST_IDLE)) / HG_LAG;
+    for(int ph = 0; ph < 3; ++ph) {
+      const int evph = p.state == ST_SW_SCAT_END ? 1 : (p.state == ST_SW_ABS_END ? 2 : 0);
+      if(p.state != ST_IDLE && p.state != ST_TRACE && p.state != ST_DONE && evph == ph)
+        path_event<V>(p, e, T.scenes[p.si], T.reqs[e.ri]);
+      const int trph = p.tr.kind != TK_TRANS ? 0 : (p.tr.prop == HG_KA ? 1 : 2);
+      uint32_t it = 0;
+      for(;; ++it) {
+        const bool act = p.state == ST_TRACE && trph == ph;
+        const unsigned m = __ballot_sync(0xffffffffu, act);
+        const uint32_t na = (uint32_t)__popc(m);
+        if(!na || (it && na <= lag)) break;
+        bool walk = false;
+        if(act) {
+          trace_enter(p.tr, T.scenes[p.si]);
+          /* an absorption trace crosses one merged leaf most often */
+          walk = (ph != 1 || it) && p.tr.has_cloud && p.tr.region == 1 && walk_fits(p.tr, T.scenes[p.si]);
+        }
+        cell_walk<V>(p, T.scenes, walk);
+        if(act && p.state == ST_TRACE) trace_step<V>(p, T.scenes[p.si]);
       }
     }
-    if(!__any_sync(0xffffffffu, p.state != ST_IDLE)) break;
-    if(p.state != ST_IDLE) {
-      const DRequest& R = T.reqs[p.ri];
-      const DScene& S = T.scenes[p.si];
-      if(p.state != ST_TRACE && p.state != ST_DONE) {
-        path_event<V>(p, S, R);
-        seg += p.c_seg; node += p.c_node; tc += p.c_tc;
-        p.c_seg = p.c_node = p.c_tc = 0;
-      }
-      if(p.state == ST_TRACE) {
-        trace_step<V>(p, S);
-      } else if(p.state == ST_DONE) {
-        accumulate_b(p, R);
-        count_grid(T.cnt, p);
-        real += (p.flags & (PF_REJECTED | PF_FAILED)) ? 0 : 1;
-        fail += (p.flags & PF_FAILED) ? 1 : 0;
-        seg += p.c_seg; node += p.c_node; tc += p.c_tc;
-        p.c_seg = p.c_node = p.c_tc = 0;
-        p.state = ST_IDLE;
-      }
+    if(p.state == ST_DONE) {
+      accumulate_b(p, e.weight, T.reqs[e.ri]);
+      count_grid(T.cnt, p);
+      atomicAdd(&sums[0], (unsigned long long)p.c_seg);
+      if(p.c_node) atomicAdd(&sums[1], (unsigned long long)p.c_node);
+      atomicAdd(&sums[2], (unsigned long long)p.c_tc);
+      if(!(p.flags & (PF_REJECTED | PF_FAILED))) atomicAdd(&sums[3], 1ull);
+      if(p.flags & PF_FAILED) atomicAdd(&sums[4], 1ull);
+      p.c_seg = p.c_node = p.c_tc = 0;
+      p.state = ST_IDLE;
     }
   }
-  seg += p.c_seg; node += p.c_node; tc += p.c_tc;
-  flush_counts(T.cnt, seg, node, tc, real, fail);
+  __syncthreads();
+  if(threadIdx.x == 0) {
+    Counters* c = (Counters*)T.cnt;
+    atomicAdd(&c->seg, sums[0]);
+    atomicAdd(&c->node, sums[1]);
+    atomicAdd(&c->tc, sums[2]);
+    atomicAdd(&c->real, sums[3]);
+    atomicAdd(&c->fail, sums[4]);
+  }
 }
 
 size_t
@@ -573,7 +653,7 @@ wave_reserve(WaveBufs& B, uint32_t P)
 namespace {
 
 using WaveEventFn = void (*)(WTables, uint32_t, int);
-using WaveFinishFn = void (*)(WTables, int);
+using WaveFinishFn = void (*)(WTables, int, uint32_t);
 WaveEventFn
 wave_event_fn(uint32_t v)
 {
@@ -596,7 +676,7 @@ struct WaveLaunch {
   /* the event and tail kernels of the tables' scenes (with or without the
    * ground-mesh queries) */
   void (*ev)(WTables, uint32_t, int) = nullptr;
-  void (*fi)(WTables, int) = nullptr;
+  void (*fi)(WTables, int, uint32_t) = nullptr;
 };
 
 cudaError_t
@@ -608,7 +688,7 @@ wave_params(const PTables& T, const htrdr_gpu_tuning& tun, int device, WaveLaunc
   L.ev = wave_event_fn(T.variant);
   L.fi = wave_finish_fn(T.variant);
   L.tb = tun.block_size ? tun.block_size : 256;
-  L.fi_smem = L.smem;
+  L.fi_smem = L.smem + finish_event_bytes();
   cudaError_t e;
   if(L.smem > 48 * 1024) {
     if((e = cudaFuncSetAttribute(L.ev, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem)))
@@ -623,13 +703,23 @@ wave_params(const PTables& T, const htrdr_gpu_tuning& tun, int device, WaveLaunc
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ev_per_sm, L.ev, 128, L.smem);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&tr_per_sm, k_wave_trace, (int)L.tb, L.smem);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fi_per_sm, L.fi, (int)L.tb, L.fi_smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fi_per_sm, L.fi, (int)(32 * HG_FINISH_WARPS), L.fi_smem);
   if(tun.blocks_per_sm) tr_per_sm = std::min(tr_per_sm, (int)tun.blocks_per_sm);
   L.ev_grid = (unsigned)(nsm * std::max(ev_per_sm, 1));
   L.tr_grid = (unsigned)(nsm * std::max(tr_per_sm, 1));
   L.fi_grid = (unsigned)(nsm * std::max(fi_per_sm, 1));
-  L.tail = tun.wave_tail ? tun.wave_tail : 4ull * L.fi_grid * L.tb;
+  L.tail = tun.wave_tail ? tun.wave_tail : 16ull * L.fi_grid * HG_FINISH_WARPS;
   return cudaSuccess;
+}
+
+/* The finishing kernel on some `paths': spread over all its warps */
+void
+launch_finish(const WTables& W, const WaveLaunch& L, uint64_t paths, cudaStream_t st)
+{
+  const uint64_t warps = (uint64_t)L.fi_grid * HG_FINISH_WARPS;
+  const uint64_t cap = (paths + warps - 1) / warps;
+  L.fi<<<L.fi_grid, 32 * HG_FINISH_WARPS, L.fi_smem, st>>>(W, L.in_smem,
+                                                           (uint32_t)std::min<uint64_t>(std::max<uint64_t>(cap, 1), 32));
 }
 
 WTables
@@ -675,11 +765,14 @@ launch_wavefront(const PTables& T, const htrdr_gpu_tuning& tun, WaveBufs& B, int
   WTables W = wave_tables(T, tun, B, false);
   W.P = P; /* the buffers may hold more slots than this run uses */
 
-  /* a run too small to fill the stages is all tail: the megakernel takes the
-   * whole queue */
-  if(P < L.tail) {
+  /* A run too small to fill the stages is all tail: the finishing kernel takes
+   * the whole queue.  So is any run with shortwave requests: 128 ms against 31
+   * for the stages and their tail on a flux map of 88 000 realisations, 750
+   * against 325 on a batch of 32 images.  Longwave walks are short and run
+   * whole in the trace stage: 18 ms against 27 on a flux map. */
+  if(P < L.tail || (T.variant & HV_SW)) {
     k_wave_init<<<1, 32, 0, st>>>(W, 0u);
-    L.fi<<<L.fi_grid, L.tb, L.fi_smem, st>>>(W, L.in_smem);
+    launch_finish(W, L, T.total, st);
     note_launches(2);
     return cudaGetLastError();
   }
@@ -707,7 +800,7 @@ launch_wavefront(const PTables& T, const htrdr_gpu_tuning& tun, WaveBufs& B, int
       const uint32_t live = hctl[(k - 1) & 1].n_live[0];
       if(live == 0) break;  /* chunk k runs empty stages */
       if(live < L.tail) {   /* after chunk k, the megakernel finishes list 0 */
-        L.fi<<<L.fi_grid, L.tb, L.fi_smem, st>>>(W, L.in_smem);
+        launch_finish(W, L, live, st);
         note_launches(1);
         return cudaGetLastError();
       }
@@ -766,7 +859,7 @@ wave_serve_finish(const PTables& T, const htrdr_gpu_tuning& tun, WaveBufs& B, in
   cudaError_t e = wave_params(T, tun, device, L);
   if(e) return e;
   const WTables W = wave_tables(T, tun, B, true);
-  L.fi<<<L.fi_grid, L.tb, L.fi_smem, st>>>(W, L.in_smem);
+  launch_finish(W, L, L.tail, st);
   k_wave_clamp<<<1, 32, 0, st>>>(W);
   note_launches(2);
   if((e = cudaGetLastError())) return e;

@@ -697,6 +697,28 @@ sub_tau(double ts, double l, double k)
   return fma(-l, k, ts);
 }
 
+/* Whether a tentative collision of a free path at a site is a real one (r in
+ * [0, 1) decides): its site and event are then the trace's */
+template <unsigned V>
+__device__ __forceinline__ bool
+real_collision(PathTrace& p, const DScene& S, int cell, int layer, float kmax, float r)
+{
+  Trace& T = p.tr;
+  const float ks = site_k(S, cell, layer, p.band, p.q, HG_KS, 3);
+  const float ps = ks / kmax;
+  if((V & HV_SW) && (!(V & HV_LW) || T.kind == TK_SCATTER)) {
+    if(!(r < ps)) return false;
+  } else {
+    const float ka = site_k(S, cell, layer, p.band, p.q, HG_KA, 3);
+    const float pa = ka / kmax;
+    if(!(r < pa + ps)) return false;
+    T.event = r < pa ? 0 : 1;
+  }
+  T.site_cell = cell;
+  T.site_layer = layer;
+  return true;
+}
+
 /* The hit filters (..._sw.c:73-217, ..._lw.c:64-135) on voxel [d0, d1].
  * Returns true when the traversal stops (real collision). */
 template <unsigned V>
@@ -707,7 +729,6 @@ voxel_filter(PathTrace& p, const DScene& S, float d0, float d1, float kmin, floa
   Trace& T = p.tr;
   /* the kinds the variant can meet (a LW-only variant meets TK_LW alone) */
   const bool trans = (V & HV_SW) && T.kind == TK_TRANS;
-  const bool scat = (V & HV_SW) && (!(V & HV_LW) || T.kind == TK_SCATTER);
   /* the traversed distance is carried in FP64 inside the voxel so that tiny
    * free paths still advance it far from the origin */
   double tc = (double)d0;
@@ -734,23 +755,7 @@ voxel_filter(PathTrace& p, const DScene& S, float d0, float d1, float kmin, floa
       k = fminf(fmaxf(k, kmin), kmax);
       if((double)r < ((double)k - (double)kmin) / kt) return true;
     } else {
-      const float ks = site_k(S, cell, layer, p.band, p.q, HG_KS, 3);
-      const float ps = ks / kmax;
-      int event = 2;
-      if(scat) {
-        if(r < ps) event = T.event; /* a scattering: the event field is the LW walk's */
-        else event = 3;
-      } else {
-        const float ka = site_k(S, cell, layer, p.band, p.q, HG_KA, 3);
-        const float pa = ka / kmax;
-        event = r < pa ? 0 : (r < pa + ps ? 1 : 3);
-      }
-      if(event != 3) {
-        T.event = (uint8_t)event;
-        T.site_cell = cell;
-        T.site_layer = layer;
-        return true;
-      }
+      if(real_collision<V>(p, S, cell, layer, kmax, r)) return true;
     }
     T.Ts = p.rng.exp1();
   }

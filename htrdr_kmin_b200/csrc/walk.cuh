@@ -63,7 +63,7 @@ walk_fits(const Trace& T, const DScene& S)
  * with a loop of ~75 instructions and the x axis consecutive in the grid,
  * 325 ms with the axis nearest to the sun consecutive, 317 ms with this loop;
  * 1024 realisations (all latency) 5.1 ms before it, 4.65 ms with it. */
-template <bool Trans>
+template <unsigned V, bool Trans>
 __device__ __forceinline__ void
 cell_walk(PathTrace& p, const DScene* scenes, bool run)
 {
@@ -92,81 +92,105 @@ cell_walk(PathTrace& p, const DScene* scenes, bool run)
   const float re = T.cb1;
   float t = T.t;
   double td = (double)t, ts = T.Ts, tmin = T.Tmin;
-  uint32_t n = 0;
-  bool out = false, black = false, go;
-  do {
-    const float te = fminf(tx, fminf(ty, tz));
-    const bool ax = tx == te, ay = !ax && ty == te;
-    uint32_t cn = ci + (uint32_t)(ax ? ix : (ay ? iy : iz));
-    int kn = (ax ? kx : (ay ? ky : kz)) - 1;
-    out = te >= re;
-    int turn = 0; /* tiles crossed */
-    if(kn < 0) { /* the border */
-      if(repeat && (ax || ay)) {
-        kn = (ax ? nx : ny) - 1;
-        cn -= (uint32_t)((kn + 1) * (ax ? ix : iy));
-        turn = (ax ? ux : uy) ? 1 : -1;
+  uint32_t n = 0, nulls = 0;
+  bool out = false, black = false, hit = false, skip = false;
+  for(;;) {
+    bool go, meet = false; /* meet: a tentative collision of a free path */
+    do {
+      const float te = fminf(tx, fminf(ty, tz));
+      const bool ax = tx == te, ay = !ax && ty == te;
+      uint32_t cn = ci + (uint32_t)(ax ? ix : (ay ? iy : iz));
+      int kn = (ax ? kx : (ay ? ky : kz)) - 1;
+      out = te >= re;
+      int turn = 0; /* tiles crossed */
+      if(kn < 0) { /* the border */
+        if(repeat && (ax || ay)) {
+          kn = (ax ? nx : ny) - 1;
+          cn -= (uint32_t)((kn + 1) * (ax ? ix : iy));
+          turn = (ax ? ux : uy) ? 1 : -1;
+        } else {
+          out = true;
+        }
+      }
+      float2 nm = mm;
+      if(!out) nm = __ldg(maj + cn);
+      /* the voxel's filter; a segment that rounding turned round is left to
+       * trace_step() */
+      const double e = (double)fminf(te, re);
+      const double l = e - td;
+      bool pass = __float_as_int(mm.y) >= 0 && te >= t;
+      if(Trans) {
+        const double tn = fma(l, (double)mm.x, tmin);
+        double sn = ts;
+        /* the filter looks at the transmissivity before the collisions */
+        black = pass && tn >= HG_TMIN_ZERO;
+        if(mm.x != mm.y) { /* null collisions: not where a cell overlaps one gas layer */
+          const double k = (double)mm.y - (double)mm.x;
+          sn = sub_tau(ts, l, k);
+          if(!(ts > __dmul_rn(l, k))) pass = false;
+        } else if(!(ts > 0.0)) {
+          pass = false;
+        }
+        if(pass || black) { tmin = tn; ts = sn; }
       } else {
-        out = true;
+        const double k = (double)mm.y;
+        const bool far = skip || ts > __dmul_rn(l, k);
+        meet = pass && !far && te > t;
+        if(pass && far && !skip) ts = sub_tau(ts, l, k);
+        pass = pass && !meet;
+        skip = false;
       }
-    }
-    float2 nm = mm;
-    if(!out) nm = __ldg(maj + cn);
-    /* the voxel's filter; a segment that rounding turned round is left to
-     * trace_step() */
-    const double e = (double)fminf(te, re);
-    const double l = e - td;
-    bool pass = __float_as_int(mm.y) >= 0 && te >= t;
-    if(Trans) {
-      const double tn = fma(l, (double)mm.x, tmin);
-      double sn = ts;
-      if(mm.x != mm.y) { /* null collisions: not where a cell overlaps one gas layer */
-        const double k = (double)mm.y - (double)mm.x;
-        sn = sub_tau(ts, l, k);
-        if(!(ts > __dmul_rn(l, k))) pass = false;
-      } else if(!(ts > 0.0)) {
-        pass = false;
-      }
-      /* the filter looks at the transmissivity before the collisions */
-      black = __float_as_int(mm.y) >= 0 && te >= t && tn >= HG_TMIN_ZERO;
-      if(pass || black) { tmin = tn; ts = sn; }
-    } else {
-      const double k = (double)mm.y;
-      pass = pass && ts > __dmul_rn(l, k);
-      if(pass) ts = sub_tau(ts, l, k);
-    }
-    if(pass || black) ++n;
-    go = pass && !black && !out;
-    if(go) {
-      if(ax) {
-        gx += sx; kx = kn; T.tile[0] += turn;
-        tx = cell_plane(gx, S.cell[0], S.lower[0], T.o.x, T.inv.x);
-      } else if(ay) {
-        gy += sy; ky = kn; T.tile[1] += turn;
-        ty = cell_plane(gy, S.cell[1], S.lower[1], T.o.y, T.inv.y);
-      } else {
-        gz += sz; kz = kn;
-        tz = cell_plane(gz, S.cell[2], S.lower[2], T.o.z, T.inv.z);
-      }
-      ci = cn;
-      t = te;
-      td = e;
-      mm = nm;
-    } else {
+      if(pass || black) ++n;
+      go = pass && !black && !out;
       out = out && pass;
+      if(go) {
+        if(ax) {
+          gx += sx; kx = kn; T.tile[0] += turn;
+          tx = cell_plane(gx, S.cell[0], S.lower[0], T.o.x, T.inv.x);
+        } else if(ay) {
+          gy += sy; ky = kn; T.tile[1] += turn;
+          ty = cell_plane(gy, S.cell[1], S.lower[1], T.o.y, T.inv.y);
+        } else {
+          gz += sz; kz = kn;
+          tz = cell_plane(gz, S.cell[2], S.lower[2], T.o.z, T.inv.z);
+        }
+        ci = cn;
+        t = te;
+        td = e;
+        mm = nm;
+        nulls = 0;
+      }
+    } while(go && n < HG_WALK_STEPS - 64u);
+    T.c[0] = (uint32_t)(ux ? nx - 1 - kx : kx);
+    T.c[1] = (uint32_t)(uy ? ny - 1 - ky : ky);
+    T.c[2] = (uint32_t)(uz ? nz - 1 - kz : kz);
+    if(Trans || !meet) break;
+    /* the lanes that met a collision, together: the voxel_filter() of a cell */
+    if(nulls >= HG_MAX_NULL) { p.flags |= PF_FAILED; skip = true; continue; }
+    const double tc = td + ts / (double)mm.y;
+    T.tcur = (float)tc;
+    if(tc > (double)HG_MAX_DIST) { skip = true; continue; }
+    const int cell = (int)((T.c[2] * S.def[1] + T.c[1]) * S.def[0] + T.c[0]);
+    const int layer = cell_layer(S, (int)T.c[2], fmaf(T.d.z, T.tcur, T.o.z));
+    ++p.c_tc;
+    const float r = p.rng.uf();
+    if(real_collision<V>(p, S, cell, layer, mm.y, r)) {
+      ++n;
+      hit = true;
+      break;
     }
-  } while(go && n < HG_WALK_STEPS - 64u);
+    ts = p.rng.exp1(); /* a null one: on from there */
+    td = tc;
+    ++nulls;
+  }
   p.c_seg += n;
   p.c_grid += 9u * n;
   T.steps += n;
   T.Ts = ts;
   if(Trans) T.Tmin = tmin;
   T.t = t;
-  T.c[0] = (uint32_t)(ux ? nx - 1 - kx : kx);
-  T.c[1] = (uint32_t)(uy ? ny - 1 - ky : ky);
-  T.c[2] = (uint32_t)(uz ? nz - 1 - kz : kz);
   T.start = 0;
-  if(black) trace_finish(p, true);
+  if(black || hit) trace_finish(p, true);
   else if(out) region_leave(p);
 }
 

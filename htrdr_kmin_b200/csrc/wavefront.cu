@@ -570,8 +570,8 @@ k_wave_finish(WTables W, int tables_in_smem, uint32_t cap)
           /* an absorption trace crosses one merged leaf most often */
           walk = (ph != 1 || it) && p.tr.has_cloud && p.tr.region == 1 && walk_fits(p.tr, T.scenes[p.si]);
         }
-        if(ph == 0) cell_walk<false>(p, T.scenes, walk);
-        else if(V & HV_SW) cell_walk<true>(p, T.scenes, walk);
+        if(ph == 0) cell_walk<V, false>(p, T.scenes, walk);
+        else if(V & HV_SW) cell_walk<V, true>(p, T.scenes, walk);
         __syncwarp();
         if(act && p.state == ST_TRACE) trace_step<V>(p, T.scenes[p.si]);
       }

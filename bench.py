@@ -10,8 +10,7 @@ realisations so that one step takes seconds (at full ranges one request holds
 up to 10^9 realisations).  A step renders the whole mix.
 
 * value: Mrealisations/s of the mix rendered in one launch of the work-queue
-  engine the autotuner picks (its wavefront tail threshold timed on the full
-  mix), outputs in HBM, scenes resident; the K steps timed between two CUDA
+  engine with the block size the autotuner picks, outputs in HBM, scenes resident; the K steps timed between two CUDA
   events that bracket them (the host's share of each call included), max
   over ranks.
 * plain_gpu / batched_vs_plain: the same requests one at a time through the
@@ -107,11 +106,8 @@ def parse_tuning(api, text: str):
 def tuning_dict(t, source: str) -> dict:
     d = {"engine": {0: "persistent", 2: "wavefront", 3: "sorted"}.get(t.engine, str(t.engine)),
          "block_size": t.block_size}
-    if t.engine == 2:
-        d.update(trace_budget=t.trace_budget or 256, wave_slots=t.wave_slots or "auto",
-                 wave_tail=t.wave_tail or "auto", tail_regroup_period=t.regroup_period)
-    else:
-        d.update(queue_chunk=t.queue_chunk, regroup_period=t.regroup_period)
+    if t.engine == 3:
+        d.update(regroup_period=t.regroup_period)
     d["from"] = source
     return d
 
@@ -778,14 +774,13 @@ def measure(args, api, su: "Setup", desc: str, tuning, tuning_src: str, rank: in
         step_ms, e2e_ms = float(t[0]), float(t[1])
 
     last = stats[-1]
-    wave = tuning.engine == api.ENGINE_WAVEFRONT
     reals = last.realisations
     kms = float(np.mean(kernel_ms))
     alg_bytes = alg_bytes_of(last)
     peak, peak_kind = peaks()
     achieved = alg_bytes / (kms * 1e-3) / 1e9
-    kernel = "wavefront" if wave else ("k_sorted" if tuning.engine == api.ENGINE_SORTED else "k_persistent")
-    traffic, traffic_src = traffic_per_launch(traffic_key or kernel, alg_bytes)
+    kernel = "k_sorted" if tuning.engine == api.ENGINE_SORTED else "k_step"
+    traffic, traffic_src = traffic_per_launch(traffic_key or ("wavefront" if kernel == "k_step" else kernel), alg_bytes)
     out_bytes = sum(d.numel() for d in su.dev)
     line = {
         "value": world * reals / (step_ms * 1e-3) / 1e6, "ms_per_step": step_ms,
@@ -805,7 +800,7 @@ def measure(args, api, su: "Setup", desc: str, tuning, tuning_src: str, rank: in
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": traffic, "traffic_source": traffic_src,
                      "peak_kind": peak_kind,
-                     "kernel": "k_wave_event + k_wave_trace + k_wave_finish" if wave else kernel,
+                     "kernel": kernel,
                      "alg_bytes_per_launch": int(alg_bytes), "kernel_ms": kms},
         "plain_gpu": {"value": reals / (plain_ms * 1e-3) / 1e6, "unit": UNIT, "kernel": "k_plain",
                       "kernel_ms": plain_ms, "launches": n},
@@ -820,36 +815,17 @@ def measure(args, api, su: "Setup", desc: str, tuning, tuning_src: str, rank: in
     return line, gpu_maps, stats
 
 
-TAILS = (25000, 50000, 100000, 200000)
-
-
 def pick_tuning(args, api, su: "Setup", name: str):
     """Tuning of the batched engine: the command line's, else the autotuner's
     (on the mix at 1/8 of its realisations per pixel for mix_full, so that its
-    28 candidate runs stay short).  The tail threshold of a wavefront pick is
-    then timed on the full mix: at 1/8 of the work the longest walks, which
-    the threshold is about, weigh eight times as much."""
+    candidate runs stay short)."""
     if args.tuning:
         return parse_tuning(api, args.tuning), "command line"
     if name != "mix_full":
         tuning, _ = api.autotune(su.items_dev)
         return tuning, "autotuner"
     tuning, _ = api.autotune(su.reduced_items(8))
-    src = "autotuner (on the same mix at 1/8 of the realisations per pixel)"
-    if tuning.engine != api.ENGINE_WAVEFRONT:
-        return tuning, src
-    L = api.lib()
-    best = None
-    for tail in TAILS:
-        t = api.Tuning(*[getattr(tuning, f) for f, _ in api.Tuning._fields_])
-        t.wave_tail = tail
-        st = api.Stats()
-        res = L.htrdr_gpu_draw_maps_batched_device(su.items_dev, su.n, C.byref(t), C.byref(st))
-        if res != 0:
-            raise api.HtrdrError("batched_device", res, L.htrdr_gpu_last_error().decode())
-        if best is None or st.kernel_ms < best[0]:
-            best = (st.kernel_ms, t)
-    return best[1], src + f", tail threshold timed on the full mix ({', '.join(map(str, TAILS))})"
+    return tuning, "autotuner (on the same mix at 1/8 of the realisations per pixel)"
 
 
 def main():
@@ -899,7 +875,7 @@ def main():
     tuning, src = pick_tuning(args, api, su, args.workload)
     fields, gpu_maps, _ = measure(args, api, su, desc, tuning, src, rank, world, dist,
                                   traffic_key="wavefront_lw" if (args.workload == "lw_flux"
-                                                                 and tuning.engine == api.ENGINE_WAVEFRONT) else "")
+                                                                 and tuning.engine != api.ENGINE_SORTED) else "")
 
     line = {"metric": METRIC, "value": fields.pop("value"), "unit": UNIT, "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": fields.pop("ms_per_step"),
@@ -942,7 +918,7 @@ def main():
         t2, src2 = pick_tuning(args, api, su2, "lw_flux") if not args.tuning else (
             api.mode_tuning(S.MODE_FLUX_LW), "mode default")
         f2, _, _ = measure(args, api, su2, desc2, t2, src2, rank, world, dist, clocks=False,
-                           traffic_key="wavefront_lw" if t2.engine == api.ENGINE_WAVEFRONT else "")
+                           traffic_key="wavefront_lw" if t2.engine != api.ENGINE_SORTED else "")
         line["lw_flux"] = {k: f2[k] for k in ("value", "ms_per_step", "e2e", "plain_gpu",
                                               "batched_vs_plain", "roofline", "segments_per_s")}
         line["lw_flux"]["unit"] = UNIT

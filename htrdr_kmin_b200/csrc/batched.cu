@@ -1,27 +1,19 @@
 /* Batched engine: many draw_map requests (images, flux maps, spectral
- * domains, scenes) in ONE persistent kernel fed by a device work queue.
+ * domains, scenes) in ONE launch fed by a device work queue.
  *
  * A launch covers items -- ranges of realisations of requests -- whose
  * realisations form one index space (item-major, realisation-major inside a
- * request).  Each resident thread owns one path slot; when its path ends it
- * takes the next realisation from its private chunk of the queue, refilled
- * `queue_chunk' realisations at a time by one warp-aggregated atomic.  Paths
- * of very different lengths therefore never leave lanes idle while work
- * remains (path regeneration), and the weight of each realisation is the same
- * as in the one-thread-per-realisation kernel because both run the same state
- * machine on the same stream.
- *
- * Lanes are regrouped by warp ballot: lanes whose trace ended (scattering
- * events, sun sampling, accumulation) and idle lanes (new realisations) wait
- * and are served together once every `regroup_period' voxel steps, or as soon
- * as no lane of the warp is tracing, so that the long sampling code runs with
- * many lanes at once while the tracing lanes keep stepping.
+ * request).  The step loop (step.cuh) runs them: each resident thread owns one
+ * path and takes the next realisation when it ends.  Paths of very different
+ * lengths therefore never leave lanes idle while work remains (path
+ * regeneration), and the weight of each realisation is the same as in the
+ * one-thread-per-realisation kernel because both run the same state machine on
+ * the same stream.  The block-sorted kernel, kept as an option, regroups the
+ * paths of a block by stage at every step instead.
  *
  * Entry points: one-shot htrdr_gpu_draw_maps_batched(_device), the reusable
  * htrdr_gpu_batch_* object whose launch sequence is captured once in a CUDA
- * graph and replayed, and the autotuner.  The one-shot entry points and the
- * autotuner also run the same items on the wavefront engine (wavefront.cu)
- * when the tuning selects it. */
+ * graph and replayed, and the autotuner. */
 #include "engine.cuh"
 
 #include <algorithm>
@@ -30,90 +22,6 @@
 #include <cstring>
 
 namespace hg {
-
-/* The persistent loop over one lane's path `p' (in registers or in shared
- * memory: see k_persistent) */
-template <unsigned V>
-__device__ __forceinline__ void
-persistent_loop(PTables& T, Path& p)
-{
-  const unsigned lane = threadIdx.x & 31u;
-  p.state = ST_IDLE;
-  p.flags = 0;
-  p.c_seg = p.c_node = p.c_tc = 0;
-  p.ri = p.si = 0;             /* request and scene of the current path */
-  uint64_t wcur = 0, wend = 0; /* private chunk of the queue */
-  bool drained = false;
-  unsigned long long seg = 0, node = 0, tc = 0, real = 0, fail = 0;
-  const uint32_t period = T.regroup_period > 1 ? T.regroup_period : 1;
-
-  for(uint32_t it = 0;; ++it) {
-    const unsigned tmask = __ballot_sync(0xffffffffu, p.state == ST_TRACE);
-    if(tmask && (it % period) != 0) { /* not a regrouping step: tracing lanes only */
-      if(p.state == ST_TRACE) trace_step<V>(p, T.scenes[p.si]);
-      continue;
-    }
-    /* refill the private chunk of lanes that are idle with nothing left */
-    const bool need = p.state == ST_IDLE && wcur >= wend && !drained;
-    const unsigned m = __ballot_sync(0xffffffffu, need);
-    if(m) {
-      const unsigned leader = __ffs(m) - 1;
-      unsigned long long base = 0;
-      if(lane == leader) base = atomicAdd(T.next, (unsigned long long)__popc(m) * T.chunk);
-      base = __shfl_sync(0xffffffffu, base, leader);
-      if(need) {
-        const unsigned rank = __popc(m & ((1u << lane) - 1u));
-        wcur = base + (unsigned long long)rank * T.chunk;
-        wend = wcur + T.chunk;
-        if(wend > T.total) wend = T.total;
-        if(wcur >= T.total) { drained = true; wcur = wend = T.total; }
-      }
-    }
-    if(p.state == ST_IDLE && wcur < wend) path_assign(p, p.ri, T, wcur++);
-    if(!__any_sync(0xffffffffu, p.state != ST_IDLE)) break;
-    if(p.state != ST_IDLE) {
-      const DRequest& R = T.reqs[p.ri];
-      const DScene& S = T.scenes[p.si];
-      if(p.state != ST_TRACE && p.state != ST_DONE) {
-        path_event<V>(p, p, S, R);
-        seg += p.c_seg; node += p.c_node; tc += p.c_tc;
-        p.c_seg = p.c_node = p.c_tc = 0;
-      }
-      if(p.state == ST_TRACE) {
-        trace_step<V>(p, S);
-      } else if(p.state == ST_DONE) {
-        accumulate_b(p, p.weight, R);
-        count_grid(T.cnt, p);
-        real += (p.flags & (PF_REJECTED | PF_FAILED)) ? 0 : 1;
-        fail += (p.flags & PF_FAILED) ? 1 : 0;
-        seg += p.c_seg; node += p.c_node; tc += p.c_tc;
-        p.c_seg = p.c_node = p.c_tc = 0;
-        p.state = ST_IDLE;
-      }
-    }
-  }
-  seg += p.c_seg; node += p.c_node; tc += p.c_tc;
-  flush_counts(T.cnt, seg, node, tc, real, fail);
-}
-
-template <unsigned V>
-__global__ void __maxnreg__(HG_PERSIST_MAXNREG)
-k_persistent(PTables T, int tables_in_smem)
-{
-  /* the scene and request views are read on every step: keep them in shared
-   * memory when they fit (one copy per block), after the block's paths when
-   * these live there too */
-  extern __shared__ __align__(16) unsigned char smem[];
-  if constexpr(persistent_smem_paths(V)) {
-    PathSlot* slots = (PathSlot*)smem;
-    if(tables_in_smem) tables_to_smem(T, smem + path_slots_bytes(blockDim.x));
-    persistent_loop<V>(T, slots[threadIdx.x].p);
-  } else {
-    if(tables_in_smem) tables_to_smem(T, smem);
-    Path p;
-    persistent_loop<V>(T, p);
-  }
-}
 
 template <unsigned V>
 __global__ void __maxnreg__(HG_PERSIST_MAXNREG)
@@ -127,14 +35,8 @@ k_sorted(PTables T, int tables_in_smem)
   sorted_loop<V>(T, slots, lists);
 }
 
-using PersistentFn = void (*)(PTables, int);
-static PersistentFn
-persistent_fn(uint32_t v)
-{
-  HG_PICK_VARIANT(v, k_persistent)
-}
-
-static PersistentFn
+using SortedFn = void (*)(PTables, int);
+static SortedFn
 sorted_fn(uint32_t v)
 {
   HG_PICK_VARIANT(v, k_sorted)
@@ -149,18 +51,14 @@ valid_tuning(const htrdr_gpu_tuning& t)
 }
 
 cudaError_t
-launch_persistent(const PTables& T, uint32_t block_size, uint32_t blocks_per_sm, int device,
-                  cudaStream_t st, bool sorted)
+launch_sorted(const PTables& T, uint32_t block_size, uint32_t blocks_per_sm, int device, cudaStream_t st)
 {
   static_assert(sizeof(DScene) % 4 == 0 && sizeof(DRequest) % 4 == 0, "word copies");
   if(!T.total) return cudaSuccess;
   const size_t tables = ((T.nscenes * sizeof(DScene) + 15) & ~(size_t)15) + T.nreqs * sizeof(DRequest);
   const int in_smem = tables <= 96 * 1024;
-  const uint32_t v = hv_make((T.variant & HV_MESH) != 0, T.variant);
-  const size_t paths = sorted ? path_slots_bytes(block_size) + sorted_lists_bytes(block_size)
-                              : (persistent_smem_paths(v) ? path_slots_bytes(block_size) : 0);
-  const size_t smem = (in_smem ? tables : 0) + paths;
-  auto kern = sorted ? sorted_fn(v) : persistent_fn(v);
+  const size_t smem = (in_smem ? tables : 0) + path_slots_bytes(block_size) + sorted_lists_bytes(block_size);
+  auto kern = sorted_fn(T.variant);
   if(smem > 227 * 1024) return cudaErrorInvalidConfiguration; /* block too large for its paths */
   if(smem > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -191,23 +89,19 @@ single_tables_bytes()
 }
 
 cudaError_t
-launch_workqueue(const PTables& T0, const htrdr_gpu_tuning& tun, WaveBufs* wave, int device,
-                 cudaStream_t st)
+launch_workqueue(const PTables& T0, const htrdr_gpu_tuning& tun, int device, cudaStream_t st)
 {
   PTables T = T0;
   T.chunk = tun.queue_chunk;
   T.regroup_period = tun.regroup_period;
-  if(tun.engine == HTRDR_GPU_ENGINE_WAVEFRONT) {
-    if(!wave) return cudaErrorInvalidValue;
-    return launch_wavefront(T, tun, *wave, device, st);
-  }
-  return launch_persistent(T, tun.block_size, tun.blocks_per_sm, device, st,
-                           tun.engine == HTRDR_GPU_ENGINE_SORTED);
+  return tun.engine == HTRDR_GPU_ENGINE_SORTED
+    ? launch_sorted(T, tun.block_size, tun.blocks_per_sm, device, st)
+    : launch_step(T, tun.block_size, tun.blocks_per_sm, device, st);
 }
 
 cudaError_t
 launch_workqueue_single(const DScene& S, const DRequest& R, void* tables, void* cnt,
-                        const htrdr_gpu_tuning& tun, WaveBufs* wave, int device, cudaStream_t st)
+                        const htrdr_gpu_tuning& tun, int device, cudaStream_t st)
 {
   SingleTables h;
   h.scene = S;
@@ -231,18 +125,7 @@ launch_workqueue_single(const DScene& S, const DRequest& R, void* tables, void* 
   T.total = h.offsets[1];
   T.cnt = cnt;
   T.next = (unsigned long long*)((char*)cnt + 64);
-  return launch_workqueue(T, tun, wave, device, st);
-}
-
-/* Threads the persistent kernel keeps resident on the device */
-uint64_t
-persistent_capacity(uint32_t block_size, uint32_t blocks_per_sm, int device)
-{
-  int nsm = 0, per_sm = 0;
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_persistent<HV_ALL>, (int)block_size, 0);
-  if(blocks_per_sm) per_sm = std::min(per_sm, (int)blocks_per_sm);
-  return (uint64_t)std::max(per_sm, 1) * (uint64_t)nsm * block_size;
+  return launch_workqueue(T, tun, device, st);
 }
 
 /* Device buffers of a plan: tables, accumulators, counters, output staging */
@@ -291,7 +174,6 @@ struct Plan {
   bool accum_out = false; /* the items' buffers receive the accumulators */
   std::vector<size_t> item_acc_bytes;
   PTables T{};
-  WaveBufs* wave = nullptr; /* path slots of the wavefront engine (the thread's pool) */
 };
 
 static htrdr_gpu_res_T
@@ -310,7 +192,6 @@ plan_build(Plan& P, const htrdr_gpu_batch_item* items, size_t n, bool host_out,
   P.accum_out = accum_out;
   if(!cuda_ok(cudaSetDevice(device), "cudaSetDevice")) return HTRDR_GPU_RES_BAD_OP;
   P.device = device;
-  P.wave = &thread_wave(device);
   if(one_shot) P.B = &thread_plan_bufs(device);
   PlanBufs& B = *P.B;
   P.reqs.resize(n);
@@ -396,8 +277,7 @@ plan_enqueue(Plan& P, const htrdr_gpu_batch_item* items, size_t n, const htrdr_g
    * the replays */
   const unsigned evf = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
   if(ok && k0) ok = cuda_ok(cudaEventRecordWithFlags(k0, st, evf), "event");
-  if(ok) ok = cuda_ok(launch_workqueue(P.T, tun, P.wave, P.device, st),
-                      tun.engine == HTRDR_GPU_ENGINE_WAVEFRONT ? "wavefront" : "k_persistent");
+  if(ok) ok = cuda_ok(launch_workqueue(P.T, tun, P.device, st), "k_step");
   if(ok && k1) ok = cuda_ok(cudaEventRecordWithFlags(k1, st, evf), "event");
   for(size_t i = 0; ok && !P.accum_out && i < n; ++i) {
     char* dout = host_out ? (char*)P.B->d_out.ptr + P.out_off[i] : (char*)items[i].buffer;
@@ -439,38 +319,21 @@ htrdr_gpu_default_tuning(htrdr_gpu_tuning* t)
   t->wave_tail = 0;
 }
 
-/* Best tunings measured on a B200: the wavefront for every mode (long
- * multiple-scattering walks in the clouds; LW walks run whole in its trace
- * stage: LW flux map 232 Mrealisations/s against 135 for the persistent
- * megakernel).  The tail threshold is where iterations stop paying for their
- * launch and one trace's latency. */
+/* The step loop for every mode, blocks of 256 (one an SM for shortwave, two
+ * for longwave; 128 measured the same).  The other fields matter to the
+ * block-sorted engine, to serving (wave_slots) or no longer. */
 extern "C" HTRDR_GPU_API void
 htrdr_gpu_mode_tuning(int mode, htrdr_gpu_tuning* t)
 {
   if(!t) return;
   htrdr_gpu_default_tuning(t);
-  if(mode == HG_XWAVE_LW || mode == HG_FLUX_LW) {
-    t->engine = HTRDR_GPU_ENGINE_WAVEFRONT;
-    t->block_size = 256;
-    t->queue_chunk = 1;
-    t->regroup_period = 64;
-    t->trace_budget = 256;
-    t->wave_tail = 100000;
-  } else if(mode == HG_IMAGE_CIE) {
-    t->engine = HTRDR_GPU_ENGINE_WAVEFRONT;
-    t->block_size = 256;
-    t->queue_chunk = 1;
-    t->regroup_period = 16;
-    t->trace_budget = 256;
-    t->wave_tail = 100000;
-  } else {
-    t->engine = HTRDR_GPU_ENGINE_WAVEFRONT;
-    t->block_size = 256;
-    t->queue_chunk = 1;
-    t->regroup_period = 64;
-    t->trace_budget = 256;
-    t->wave_tail = 25000;
-  }
+  const bool lw = mode == HG_XWAVE_LW || mode == HG_FLUX_LW;
+  t->engine = HTRDR_GPU_ENGINE_WAVEFRONT;
+  t->block_size = 256;
+  t->queue_chunk = 1;
+  t->regroup_period = mode == HG_IMAGE_CIE ? 16 : 64;
+  t->trace_budget = 256;
+  t->wave_tail = lw || mode == HG_IMAGE_CIE ? 100000 : 25000;
 }
 
 /* `tuning' if given, else the default of the items' modes (SW/CIE if any) */
@@ -540,51 +403,23 @@ try {
 }
 HG_API_CATCH("htrdr_gpu_draw_maps_batched_accum_device")
 
-/* Autotuner: times every candidate -- persistent megakernel (block size x
- * queue chunk x regroup period) and wavefront (tail threshold x regroup
- * period of its finishing megakernel) -- on the given items (device buffers)
- * with CUDA events and returns the fastest.  Results do not depend on the
- * tuning. */
+/* Autotuner: times the step loop with every candidate block size on the given
+ * items (device buffers) with CUDA events and returns the fastest.  Results do
+ * not depend on the tuning. */
 extern "C" HTRDR_GPU_API htrdr_gpu_res_T
 htrdr_gpu_autotune(htrdr_gpu_batch_item* items, size_t n, htrdr_gpu_tuning* best, double* best_ms)
 try {
   if(!items || !n || !best) return HTRDR_GPU_RES_BAD_ARG;
-  static const uint32_t blocks[] = {96, 128, 256}; /* 96: 3 blocks of 3 warps fill 9 warps at 216 registers */
-  static const uint32_t chunks[] = {1, 4};
-  static const uint32_t periods[] = {1, 4, 16, 64};
-  static const uint32_t tails[] = {25000, 100000};
-  static const uint32_t wperiods[] = {16, 64};
+  static const uint32_t blocks[] = {64, 128, 256};
   htrdr_gpu_stats st;
   double best_t = 1e300;
-  htrdr_gpu_tuning t;
-  htrdr_gpu_default_tuning(&t);
+  htrdr_gpu_tuning t = items_tuning(items, n, nullptr);
   htrdr_gpu_res_T res = batched_impl(items, n, &t, &st, false); /* warm-up */
   if(res != HTRDR_GPU_RES_OK) return res;
-  auto time_it = [&](const htrdr_gpu_tuning& c) {
-    htrdr_gpu_res_T r = batched_impl(items, n, &c, &st, false);
-    if(r == HTRDR_GPU_RES_OK && st.kernel_ms < best_t) { best_t = st.kernel_ms; *best = c; }
-    return r;
-  };
-  for(uint32_t b : blocks) { /* persistent megakernel */
-    for(uint32_t c : chunks)
-      for(uint32_t p : periods) {
-        t.block_size = b;
-        t.queue_chunk = c;
-        t.regroup_period = p;
-        if((res = time_it(t)) != HTRDR_GPU_RES_OK) return res;
-      }
-  }
-  htrdr_gpu_default_tuning(&t);
-  t.engine = HTRDR_GPU_ENGINE_WAVEFRONT;
-  t.block_size = 256;
-  t.queue_chunk = 1;
-  t.trace_budget = 256;
-  for(uint32_t tl : tails) { /* wavefront: tail threshold x regroup period of its tail */
-    for(uint32_t p : wperiods) {
-      t.wave_tail = tl;
-      t.regroup_period = p;
-      if((res = time_it(t)) != HTRDR_GPU_RES_OK) return res;
-    }
+  for(uint32_t b : blocks) {
+    t.block_size = b;
+    if((res = batched_impl(items, n, &t, &st, false)) != HTRDR_GPU_RES_OK) return res;
+    if(st.kernel_ms < best_t) { best_t = st.kernel_ms; *best = t; }
   }
   if(best_ms) *best_ms = best_t;
   return HTRDR_GPU_RES_OK;
@@ -629,8 +464,7 @@ try {
   if(!tuning) tun.engine = HTRDR_GPU_ENGINE_PERSISTENT; /* a mode default may name the wavefront */
   if(!valid_tuning(tun)) return HTRDR_GPU_RES_BAD_ARG;
   if(tun.engine != HTRDR_GPU_ENGINE_PERSISTENT && tun.engine != HTRDR_GPU_ENGINE_SORTED) {
-    set_error("graph batches run the persistent engines (the wavefront's iteration count is "
-              "decided on the host)");
+    set_error("graph batches run the persistent engines");
     return HTRDR_GPU_RES_BAD_ARG;
   }
   auto b = new htrdr_gpu_batch();

@@ -80,9 +80,7 @@ draw_map_impl(htrdr_gpu_scene* scn, const htrdr_gpu_request* req,
     R.acc = acc;
     R.tacc = tacc;
     ok = ok && cuda_ok(launch_workqueue_single(scn->d, R, ws.tables.ptr, ws.cnt.ptr, tun,
-                                               &thread_wave(scn->device),
-                                               scn->device, st),
-                       tun.engine == HTRDR_GPU_ENGINE_WAVEFRONT ? "wavefront" : "k_persistent");
+                                               scn->device, st), "k_step");
   }
   cudaEventRecord(e2, st);
   if(!user_acc)
@@ -200,16 +198,34 @@ radiance_impl(htrdr_gpu_scene* scn, int lw, size_t n, const double* pos, const d
   }
   if(!n) return HTRDR_GPU_RES_OK;
   if(!cuda_ok(cudaSetDevice(scn->device), "cudaSetDevice")) return HTRDR_GPU_RES_BAD_OP;
-  DevArr<double> dp, dd, dw, dout;
-  DevArr<uint32_t> db, dq;
-  if(!dp.from(pos, 3 * n) || !dd.from(dir, 3 * n) || !dw.from(wlen, n) || !db.from(iband, n)
-  || !dq.from(iquad, n) || !dout.make(n))
-    return HTRDR_GPU_RES_MEM_ERR;
-  if(!cuda_ok(launch_radiance(scn->d, lw, n, dp.p(), dd.p(), dw.p(), db.p(), dq.p(), mask, seed,
-                              dout.p(), scn->stream), "k_radiance")
-  || !cuda_ok(cudaStreamSynchronize(scn->stream), "sync") || !dout.to(out, n))
-    return HTRDR_GPU_RES_UNKNOWN_ERR;
-  return HTRDR_GPU_RES_OK;
+  /* one allocation for the rays, the radiances and the counter: each of six
+   * buffers cost its allocation and, at its release, a device-wide wait */
+  DevBuf buf;
+  if(!buf.alloc(n * (8 * 8 + 2 * 4) + 16)) return HTRDR_GPU_RES_MEM_ERR;
+  double* d = (double*)buf.ptr;
+  RayArgs a;
+  a.lw = lw;
+  a.mask = mask;
+  a.seed = seed;
+  a.n = n;
+  a.next = (unsigned long long*)d;
+  a.pos = d + 2;
+  a.dir = a.pos + 3 * n;
+  a.wlen = a.dir + 3 * n;
+  a.out = d + 2 + 7 * n;
+  a.band = (const uint32_t*)(a.out + n);
+  a.iquad = a.band + n;
+  cudaStream_t st = scn->stream;
+  auto h2d = [&](const void* dst, const void* src, size_t bytes) {
+    return cuda_ok(cudaMemcpyAsync(const_cast<void*>(dst), src, bytes, cudaMemcpyHostToDevice, st), "H2D");
+  };
+  const bool ok = cuda_ok(cudaMemsetAsync(a.next, 0, 8, st), "memset") && h2d(a.pos, pos, 24 * n)
+               && h2d(a.dir, dir, 24 * n) && h2d(a.wlen, wlen, 8 * n) && h2d(a.band, iband, 4 * n)
+               && h2d(a.iquad, iquad, 4 * n)
+               && cuda_ok(launch_radiance(scn->d, a, scn->device, st), "k_radiance")
+               && cuda_ok(cudaMemcpyAsync(out, a.out, 8 * n, cudaMemcpyDeviceToHost, st), "D2H");
+  /* also after an error: the copies in flight read the caller's arrays */
+  return cuda_ok(cudaStreamSynchronize(st), "sync") && ok ? HTRDR_GPU_RES_OK : HTRDR_GPU_RES_UNKNOWN_ERR;
 }
 
 extern "C" HTRDR_GPU_API htrdr_gpu_res_T

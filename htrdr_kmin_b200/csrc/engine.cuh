@@ -1,5 +1,5 @@
-/* Device pieces shared by the work-queue engines (persistent megakernel and
- * wavefront): item lookup in the realisation index space and the FP64
+/* Device pieces shared by the work-queue engines (the step loop and the
+ * block-sorted one): item lookup in the realisation index space and the FP64
  * accumulation of a finished realisation into its request's accumulators. */
 #ifndef HTRDR_ENGINE_CUH
 #define HTRDR_ENGINE_CUH
@@ -109,9 +109,8 @@ path_assign(PathTrace& p, uint32_t& ri, const hg::PTables& T, uint64_t g)
 
 /* Takes up to n realisations from the work queue (one atomic per warp).
  * Returns the first index; *got is how many were taken (0: empty).  The head
- * may pass the queued total; the wavefront's trace stage, which takes no
- * work, clamps it back, so that work appended between chunks starts exactly
- * at the head. */
+ * may pass the queued total; the serving pool clamps it back after a launch, so
+ * that work appended between launches starts exactly at the head. */
 __device__ __forceinline__ unsigned long long
 queue_take(const hg::PTables& T, unsigned n, unsigned* got)
 {
@@ -172,20 +171,6 @@ __host__ __device__ constexpr size_t
 path_slots_bytes(uint32_t threads)
 {
   return ((size_t)threads * sizeof(PathSlot) + 15) & ~(size_t)15;
-}
-
-/* Where the persistent kernel keeps a lane's path.  LW-only launches keep it
- * in shared memory: with the path out of the registers the kernel needs ~156
- * of them instead of 216, so 12 warps fit on an SM instead of 8, and LW
- * walks are short enough that the shared-memory latency of each field access
- * costs less than the occupancy gains (1149 against 919 Mrealisations/s on
- * the LW flux map).  Shortwave walks are long and touch the path state
- * between every dependent load: they keep it in registers (in shared memory
- * the SW image ran 23 % slower). */
-__host__ __device__ constexpr bool
-persistent_smem_paths(unsigned v)
-{
-  return (v & HV_SW) == 0;
 }
 
 __device__ __forceinline__ void

@@ -145,10 +145,17 @@ cudaError_t launch_plain(const DScene& S, const DRequest& R, DAccum* acc, DAccum
                          cudaStream_t st);
 cudaError_t launch_finalize(const DRequest& R, const DAccum* acc, const DAccum* tacc,
                             void* out, size_t pitch, cudaStream_t st);
-cudaError_t launch_radiance(const DScene& S, int lw, size_t n, const double* pos,
-                            const double* dir, const double* wlen, const uint32_t* band,
-                            const uint32_t* iquad, int mask, uint32_t seed, double* out,
-                            cudaStream_t st);
+/* Rays of a radiance call (device memory); next: zeroed counter */
+struct RayArgs {
+  int lw, mask;
+  uint32_t seed;
+  size_t n;
+  const double *pos, *dir, *wlen;
+  const uint32_t *band, *iquad;
+  double* out;
+  unsigned long long* next;
+};
+cudaError_t launch_radiance(const DScene& S, const RayArgs& a, int device, cudaStream_t st);
 cudaError_t launch_find_band(const DScene& S, size_t n, const double* wlen, uint32_t* out,
                              cudaStream_t st);
 cudaError_t launch_sample_quad(const DScene& S, size_t n, const double* r, const uint32_t* band,
@@ -193,73 +200,47 @@ tables_variant(const std::vector<DScene>& scenes, const std::vector<DRequest>& r
   for(const DRequest& r : reqs) kinds |= hv_kind(r.mode);
   return hv_make(mesh, kinds);
 }
-cudaError_t launch_persistent(const PTables& T, uint32_t block_size, uint32_t blocks_per_sm,
-                              int device, cudaStream_t st, bool sorted = false);
+cudaError_t launch_sorted(const PTables& T, uint32_t block_size, uint32_t blocks_per_sm, int device,
+                          cudaStream_t st);
 bool valid_tuning(const htrdr_gpu_tuning& t);
-uint64_t persistent_capacity(uint32_t block_size, uint32_t blocks_per_sm, int device);
 /* One request on the persistent engine.  `tables' (device memory of
  * single_tables_bytes()) receives the launch's scene/request/item tables;
  * `cnt' (device, 128 bytes) holds the counters and the queue head and must be
  * zeroed before the launch. */
 size_t single_tables_bytes();
 
-/* Control block of a wavefront run (device) */
-struct WCtl {
-  uint32_t n_live[2];   /* lengths of the two live lists */
-  uint32_t fetch_event; /* next entry of the event stage's input list */
-  uint32_t fetch_trace; /* next entry of the trace stage's list */
-  uint32_t fetch_finish;/* next entry of the live list taken by the finishing megakernel */
-  uint32_t n_dead;      /* free slots on the dead list (serving) */
-  uint32_t pad[2];
-};
+/* Step loop (step.cu): all queued realisations of T in one launch */
+cudaError_t launch_step(const PTables& T, uint32_t block_size, uint32_t blocks_per_sm, int device,
+                        cudaStream_t st);
+/* Threads that launch keeps resident on the device */
+uint64_t step_capacity(uint32_t block_size, uint32_t blocks_per_sm, int device);
 
-/* Wavefront engine (wavefront.cu): path slots, live lists, control block and
- * the pinned read-back of the live count, kept between runs; `dead' holds
- * the free slots of a serving pool */
-struct WaveBufs {
-  DevBuf paths, lists, ctl, dead;
-  void* host_ctl = nullptr;
-  cudaEvent_t ev[2] = {nullptr, nullptr};
-  uint32_t P = 0;
-  WaveBufs() = default;
-  WaveBufs(const WaveBufs&) = delete;
-  WaveBufs& operator=(const WaveBufs&) = delete;
-  ~WaveBufs();
+/* Serving pool: launches that end after `ns' with their live paths saved.
+ * `paths' are read and written in turn; n[i] paths are saved in paths[i]. */
+struct StepCtl {
+  uint32_t n[2];
+  uint32_t fetch; /* next saved path to take */
+  uint32_t pad;
 };
-/* Device bytes of one path slot */
-size_t wave_slot_bytes();
-/* Path slots of the wavefront when the tuning gives none: 2^21 (940 MB).
- * Measured on a B200 (Mrealisations/s, 2^20 / 2^21 slots): full-size mix
- * 1.979 / 2.084, LW flux map 229 / 247. */
-constexpr uint32_t kDefaultWaveSlots = 1u << 21;
-/* Grow-only slot pool of the calling host thread on `device', for the calls
- * that run the wavefront engine to completion before they return (one call
- * at a time per thread): a call reuses the slots of the last one instead of
- * allocating and freeing some 460 MB of device memory and its pinned control
- * block. */
-WaveBufs& thread_wave(int device);
-cudaError_t launch_wavefront(const PTables& T, const htrdr_gpu_tuning& tun, WaveBufs& B,
-                             int device, cudaStream_t st);
-/* Serving pool of P slots driven chunk by chunk (the caller owns the queue):
- * reset = every slot free; revive = free slots join live list 0 (after work
- * was appended); chunk = an even number of event+trace iterations; finish =
- * the live paths complete in one megakernel launch, then reset.  The tail
- * threshold is the tuning's (or its default) for these launch shapes. */
-cudaError_t wave_serve_reset(WaveBufs& B, uint32_t P, cudaStream_t st);
-cudaError_t wave_serve_revive(WaveBufs& B, cudaStream_t st);
-cudaError_t wave_serve_chunk(const PTables& T, const htrdr_gpu_tuning& tun, WaveBufs& B, int device,
-                             uint32_t iterations, cudaStream_t st);
-cudaError_t wave_serve_finish(const PTables& T, const htrdr_gpu_tuning& tun, WaveBufs& B,
-                              int device, cudaStream_t st);
-uint64_t wave_serve_tail(const htrdr_gpu_tuning& tun, int device);
-/* One launch of a work-queue engine over T: persistent kernel or wavefront
- * (tun.engine; `wave' holds the wavefront's buffers) */
-cudaError_t launch_workqueue(const PTables& T, const htrdr_gpu_tuning& tun, WaveBufs* wave,
-                             int device, cudaStream_t st);
+struct StepPool {
+  uint4* paths[2];
+  StepCtl* ctl;
+  uint32_t turn, lanes;
+  uint64_t ns;
+};
+struct StepBufs {
+  DevBuf paths[2], ctl;
+  uint32_t lanes = 0; /* paths in flight at most */
+  uint32_t turn = 0;  /* paths[turn] holds the saved ones */
+};
+bool step_pool_create(StepBufs& B, uint32_t lanes, int device, cudaStream_t st);
+cudaError_t step_pool_launch(const PTables& T, StepBufs& B, uint64_t ns, uint32_t blocks_per_sm, int device,
+                             cudaStream_t st);
+/* One launch of a work-queue engine over T (tun.engine) */
+cudaError_t launch_workqueue(const PTables& T, const htrdr_gpu_tuning& tun, int device, cudaStream_t st);
 /* The same for one request; the tables are staged in `tables' */
 cudaError_t launch_workqueue_single(const DScene& S, const DRequest& R, void* tables, void* cnt,
-                                    const htrdr_gpu_tuning& tun, WaveBufs* wave, int device,
-                                    cudaStream_t st);
+                                    const htrdr_gpu_tuning& tun, int device, cudaStream_t st);
 
 }  // namespace hg
 

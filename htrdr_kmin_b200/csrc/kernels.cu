@@ -5,7 +5,7 @@
  * realisation i / npix of pixel i % npix, so the 32 lanes of a warp trace
  * neighbouring pixels and accumulate into distinct FP64 accumulators. */
 #include "internal.h"
-#include "transport.cuh"
+#include "step.cuh"
 
 namespace hg {
 
@@ -165,33 +165,73 @@ k_finalize(DRequest R, const DAccum* acc, const DAccum* tacc, char* out, size_t 
 }
 
 /*******************************************************************************
- * Batched radiance (atmosphere_compute_radiance_sw/_lw with one stream per ray)
+ * Batched radiance (atmosphere_compute_radiance_sw/_lw with one stream per
+ * ray): the step loop over the caller's rays.  A thread per ray, whose warps
+ * wait for their longest walk and run the states of 32 paths one after
+ * another, took 50 ms for 20 000 shortwave rays under a cloud.
  ******************************************************************************/
+struct RayWork {
+  const DScene* scenes;
+  const DRequest* req; /* its mode only */
+  RayArgs a;
+
+  __device__ __forceinline__ const DRequest& request(const PathEvent&) const { return *req; }
+  __device__ __forceinline__ bool stop() const { return false; }
+  __device__ __forceinline__ void save(const PathTrace&, const PathEvent&) {}
+
+  __device__ __forceinline__ bool take(bool want, PathTrace& p, PathEvent& e)
+  {
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned m = __ballot_sync(HG_FULL, want);
+    if(!m) return true;
+    const unsigned leader = __ffs(m) - 1;
+    unsigned long long i = 0;
+    if(lane == leader) i = atomicAdd(a.next, (unsigned long long)__popc(m));
+    i = __shfl_sync(HG_FULL, i, leader) + __popc(m & ((1u << lane) - 1u));
+    if(!want) return true;
+    if(i >= a.n) return false;
+    p.rng.init((uint32_t)i, a.seed, 0u, 0u);
+    e.pos = mk3((float)a.pos[3 * i], (float)a.pos[3 * i + 1], (float)a.pos[3 * i + 2]);
+    e.dir = mk3((float)a.dir[3 * i], (float)a.dir[3 * i + 1], (float)a.dir[3 * i + 2]);
+    e.org = e.pos;
+    e.rdir = e.dir;
+    e.wlen_d = a.wlen[i];
+    e.wlen = (float)a.wlen[i];
+    p.band = a.band[i];
+    p.q = __ldg(scenes[0].quad_off + p.band) + a.iquad[i];
+    e.inv_pdf = 1.0;
+    p.flags = a.lw ? PF_LW : (((a.mask & 1) ? PF_DIRECT : 0u) | ((a.mask & 2) ? PF_DIFFUSE : 0u));
+    p.c_grid = 0;
+    p.pix = (uint32_t)i; /* with ireal, the ray */
+    p.ireal = (uint32_t)(i >> 32);
+    p.state = ST_RAD_BEGIN;
+    return true;
+  }
+
+  __device__ __forceinline__ void done(const PathTrace& p, const PathEvent& e)
+  {
+    a.out[((size_t)p.ireal << 32) | p.pix] =
+      (p.flags & PF_FAILED) ? __longlong_as_double(0x7ff8000000000000ll) : e.weight;
+  }
+};
+
 template <unsigned V>
-__global__ void __launch_bounds__(128)
-k_radiance(DScene S, int lw, size_t n, const double* pos, const double* dir, const double* wlen,
-           const uint32_t* band, const uint32_t* iquad, int mask, uint32_t seed, double* out)
+__global__ void __maxnreg__(step_registers(V))
+k_radiance(DScene S, RayArgs a)
 {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if(i >= n) return;
-  DRequest R;
-  R.mode = lw ? HG_RAD_LW : HG_RAD_SW;
-  Path p;
-  p.rng.init((uint32_t)i, seed, 0u, 0u);
-  p.pos = mk3((float)pos[3 * i], (float)pos[3 * i + 1], (float)pos[3 * i + 2]);
-  p.dir = mk3((float)dir[3 * i], (float)dir[3 * i + 1], (float)dir[3 * i + 2]);
-  p.org = p.pos;
-  p.rdir = p.dir;
-  p.wlen_d = wlen[i];
-  p.wlen = (float)wlen[i];
-  p.band = band[i];
-  p.q = S.quad_off[band[i]] + iquad[i];
-  p.inv_pdf = 1.0;
-  p.flags = lw ? PF_LW : (((mask & 1) ? PF_DIRECT : 0u) | ((mask & 2) ? PF_DIFFUSE : 0u));
-  p.c_seg = p.c_node = p.c_tc = 0;
-  p.state = ST_RAD_BEGIN;
-  run_path<V>(p, S, R);
-  out[i] = (p.flags & PF_FAILED) ? __longlong_as_double(0x7ff8000000000000ll) : p.weight;
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ DScene scene;
+  __shared__ DRequest req;
+  if(threadIdx.x == 0) {
+    scene = S;
+    req.mode = a.lw ? HG_RAD_LW : HG_RAD_SW;
+  }
+  __syncthreads();
+  RayWork work{&scene, &req, a};
+  PathTrace p;
+  /* few rays are spread over all warps */
+  const size_t warps = (size_t)gridDim.x * (blockDim.x >> 5);
+  step_loop<V>(work, p, ((PathEvent*)smem)[threadIdx.x], (threadIdx.x & 31u) >= (a.n + warps - 1) / warps);
 }
 
 /*******************************************************************************
@@ -271,8 +311,7 @@ plain_fn(uint32_t v)
   HG_PICK_VARIANT(v, k_plain)
 }
 
-using RadianceFn = void (*)(DScene, int, size_t, const double*, const double*, const double*,
-                            const uint32_t*, const uint32_t*, int, uint32_t, double*);
+using RadianceFn = void (*)(DScene, RayArgs);
 static RadianceFn
 radiance_fn(uint32_t v)
 {
@@ -314,13 +353,16 @@ launch_finalize(const DRequest& R, const DAccum* acc, const DAccum* tacc, void* 
 }
 
 cudaError_t
-launch_radiance(const DScene& S, int lw, size_t n, const double* pos, const double* dir,
-                const double* wlen, const uint32_t* band, const uint32_t* iquad, int mask,
-                uint32_t seed, double* out, cudaStream_t st)
+launch_radiance(const DScene& S, const RayArgs& a, int device, cudaStream_t st)
 {
-  if(!n) return cudaSuccess;
-  auto kern = radiance_fn(hv_make(S.g_ntris != 0, lw ? HV_LW : HV_SW));
-  kern<<<nblocks(n, 128), 128, 0, st>>>(S, lw, n, pos, dir, wlen, band, iquad, mask, seed, out);
+  if(!a.n) return cudaSuccess;
+  auto kern = radiance_fn(hv_make(S.g_ntris != 0, a.lw ? HV_LW : HV_SW));
+  const unsigned threads = 128;
+  const size_t smem = step_event_bytes(threads);
+  int nsm = 0, per_sm = 0;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (int)threads, smem);
+  kern<<<(unsigned)(nsm * (per_sm > 0 ? per_sm : 1)), threads, smem, st>>>(S, a);
   return cudaGetLastError();
 }
 

@@ -49,7 +49,7 @@ struct SReq {
   int state = 0;           /* 0 pending, 1 active, 2 done */
   htrdr_gpu_res_T result = HTRDR_GPU_RES_OK;
   clk::time_point t_submit, t_done;
-  /* wavefront serving: request-table slot, scene-table slot, first chunk
+  /* pool serving: request-table slot, scene-table slot, first launch
    * whose read-back covers the request, stream-ordered buffers, and the
    * event of the map's copy to the host */
   uint32_t rslot = 0, sslot = 0;
@@ -58,7 +58,7 @@ struct SReq {
   void* out_a = nullptr;
   cudaEvent_t copied = nullptr;
   bool finishing = false;
-  /* launches of the loop (rounds or wavefront chunks) that carried the
+  /* launches of the loop (rounds, or launches of the pool) that carried the
    * request: the first with some of its realisations queued, and the last
    * before all of them were known done (UINT64_MAX: none yet) */
   uint64_t first_launch = UINT64_MAX, last_launch = 0;
@@ -133,17 +133,16 @@ struct htrdr_gpu_server {
   void loop();
   bool launch_round(Slot& s, const std::vector<SReq*>& act);
 
-  /* wavefront serving (cfg.tuning.engine == HTRDR_GPU_ENGINE_WAVEFRONT) */
+  /* pool serving (cfg.tuning.engine == HTRDR_GPU_ENGINE_WAVEFRONT) */
   struct Readback {
-    WCtl ctl;
+    StepCtl ctl;
     unsigned long long next;
     unsigned long long ndone[1]; /* [kMaxReqs] */
   };
   static constexpr uint32_t kMaxReqs = 4096, kMaxScenes = 256;
   static constexpr uint64_t kMaxItems = 1u << 20;
-  WaveBufs wave;
-  uint32_t wave_P = 0;
-  uint64_t wave_tail = 0;
+  StepBufs pool;
+  uint64_t queue_depth = 0; /* realisations kept queued */
   DevBuf w_scenes, w_reqs, w_items, w_offsets, w_cnt, w_ndone;
   void* w_rb[2] = {nullptr, nullptr}; /* pinned read-backs */
   cudaEvent_t w_ev[2] = {nullptr, nullptr}, w_ta[2] = {nullptr, nullptr}, w_tb[2] = {nullptr, nullptr};
@@ -155,7 +154,7 @@ struct htrdr_gpu_server {
                                                 * the pool may hold paths of each */
   uint64_t w_nitems = 0, w_appended = 0;       /* queue: items and realisations appended */
   std::vector<uint64_t> w_offsets_host;        /* [w_nitems + 1] */
-  bool w_pool_live = false;                    /* slots hold paths (not all free) */
+  bool w_pool_live = false;                    /* realisations queued or paths live */
   void loop_wave();
   bool wave_setup();
   bool wave_admit(SReq* r);
@@ -232,9 +231,7 @@ htrdr_gpu_server::launch_round(Slot& s, const std::vector<SReq*>& act)
   T.chunk = cfg.tuning.queue_chunk;
   T.regroup_period = cfg.tuning.regroup_period;
   ok = ok && cuda_ok(cudaEventRecord(s.e0, s.st), "event")
-          && cuda_ok(launch_persistent(T, cfg.tuning.block_size, cfg.tuning.blocks_per_sm, cfg.device, s.st,
-                                       cfg.tuning.engine == HTRDR_GPU_ENGINE_SORTED),
-                     "k_persistent")
+          && cuda_ok(launch_workqueue(T, cfg.tuning, cfg.device, s.st), "k_step")
           && cuda_ok(cudaEventRecord(s.e1, s.st), "event");
   realisations += T.total;
   s.busy = true;
@@ -350,25 +347,28 @@ htrdr_gpu_server::loop()
 }
 
 /*******************************************************************************
- * Wavefront serving: one pool of path slots fed by a growing work queue.
+ * Pool serving: one pool of paths in flight fed by a growing work queue.
  *
  * Admitted requests get a slot in a device request table and stay resident;
  * the scheduling thread appends fair-share slices of every admitted
- * request's remaining realisations to the queue (keeping about one pool of
- * realisations queued), and runs chunks of event+trace iterations.  Paths
- * that end take the next queued realisation in their slot, so requests that
- * arrive while others render start in the slots those free.  Per-request
- * counters of finished realisations, read back after every chunk, tell when
- * a request's map is complete (finalize, copy to the host buffer).  When no
- * work is queued and few paths are live, the megakernel finishes them and
- * the pool returns to all-free; a slot that finds the queue empty waits on
- * the dead list until work is appended.
+ * request's remaining realisations to the queue and launches the step loop
+ * over it, again and again.  A launch ends after kLaunchNs (or when nothing is
+ * left) and saves its live paths, which the next one resumes, spread evenly
+ * over its warps; a path that ends takes the next queued realisation, so
+ * requests that arrive while others render start in the next launch.
+ * Per-request counters of finished realisations, read back after every
+ * launch, tell when a request's map is complete (finalize, copy to the host
+ * buffer).
  ******************************************************************************/
+/* Saving and resuming a full pool takes ~20 us: 1 % of a launch */
+static constexpr uint64_t kLaunchNs = 2000000;
+
 bool
 htrdr_gpu_server::wave_setup()
 {
-  wave_P = cfg.tuning.wave_slots ? cfg.tuning.wave_slots : kDefaultWaveSlots;
-  wave_tail = wave_serve_tail(cfg.tuning, cfg.device);
+  /* enough for the lanes that go dry in two launches: a longwave flux map
+   * takes 250 000 realisations a millisecond */
+  queue_depth = cfg.tuning.wave_slots ? cfg.tuning.wave_slots : 1u << 21;
   const size_t rb = sizeof(Readback) + (kMaxReqs - 1) * sizeof(unsigned long long);
   bool ok = w_scenes.alloc(kMaxScenes * sizeof(DScene)) && w_reqs.alloc(kMaxReqs * sizeof(DRequest))
          && w_items.alloc(kMaxItems * sizeof(PItem)) && w_offsets.alloc((kMaxItems + 1) * 8)
@@ -380,7 +380,7 @@ htrdr_gpu_server::wave_setup()
   ok = ok && cuda_ok(cudaMemsetAsync(w_cnt.ptr, 0, 128, io), "memset")
           && cuda_ok(cudaMemsetAsync(w_ndone.ptr, 0, kMaxReqs * 8, io), "memset")
           && cuda_ok(cudaMemsetAsync(w_offsets.ptr, 0, 8, io), "memset")
-          && cuda_ok(wave_serve_reset(wave, wave_P, io), "wavefront pool")
+          && step_pool_create(pool, cfg.tuning.wave_slots, cfg.device, io)
           && cuda_ok(cudaStreamSynchronize(io), "sync");
   w_offsets_host.assign(1, 0);
   for(uint32_t i = kMaxReqs; i-- > 0;) w_free_rslots.push_back(i);
@@ -513,9 +513,9 @@ htrdr_gpu_server::loop_wave()
 {
   cudaSetDevice(cfg.device);
   bool failed_gpu = !wave_setup();
-  const uint32_t C = 8;       /* iterations per chunk */
-  uint64_t k = 0;             /* launches (chunks and finishes), each with a read-back */
+  uint64_t k = 0;             /* launches, each with a read-back */
   bool inflight[2] = {false, false};
+  uint32_t rb_turn[2] = {0, 0}; /* the saved paths' counter of each read-back */
   uint64_t rb_k[2] = {0, 0};  /* launch index of each read-back buffer */
   /* the queue restarts from zero between epochs: a read-back issued in an
    * earlier epoch holds the head of a queue that no longer exists */
@@ -531,7 +531,7 @@ htrdr_gpu_server::loop_wave()
     if(cudaEventElapsedTime(&ms, w_ta[b], w_tb[b]) == cudaSuccess) busy_ms += ms;
     const Readback* rb = (const Readback*)w_rb[b];
     dev_next = rb_epoch[b] == epoch ? rb->next : 0; /* else: nothing known taken yet */
-    dev_live = rb->ctl.n_live[0];
+    dev_live = rb->ctl.n[rb_turn[b]];
     for(SReq* r : active) {
       /* a read-back issued before the request was admitted holds another
        * request's count in its table slot */
@@ -575,16 +575,16 @@ htrdr_gpu_server::loop_wave()
       finish(r, r->result);
     }
   };
-  /* a chunk (or the finish) into read-back buffer b */
-  auto launch = [&](int b, bool finish_all) -> bool {
+  /* a launch into read-back buffer b */
+  auto launch = [&](int b) -> bool {
     Readback* rb = (Readback*)w_rb[b];
     const PTables T = wave_tables_now();
     const bool ok =
       cuda_ok(cudaEventRecord(w_ta[b], io), "event")
-      && (finish_all ? cuda_ok(wave_serve_finish(T, cfg.tuning, wave, cfg.device, io), "wavefront finish")
-                     : cuda_ok(wave_serve_chunk(T, cfg.tuning, wave, cfg.device, C, io), "wavefront chunk"))
+      && cuda_ok(step_pool_launch(T, pool, std::min<uint64_t>(kLaunchNs, (uint64_t)(cfg.round_target_ms * 1e6)),
+                                  cfg.tuning.blocks_per_sm, cfg.device, io), "k_step_pool")
       && cuda_ok(cudaEventRecord(w_tb[b], io), "event")
-      && cuda_ok(cudaMemcpyAsync(&rb->ctl, wave.ctl.ptr, sizeof(WCtl), cudaMemcpyDeviceToHost, io), "D2H")
+      && cuda_ok(cudaMemcpyAsync(&rb->ctl, pool.ctl.ptr, sizeof(StepCtl), cudaMemcpyDeviceToHost, io), "D2H")
       && cuda_ok(cudaMemcpyAsync(&rb->next, (char*)w_cnt.ptr + 64, 8, cudaMemcpyDeviceToHost, io), "D2H")
       && (w_nreqs == 0
           || cuda_ok(cudaMemcpyAsync(rb->ndone, w_ndone.ptr, (size_t)w_nreqs * 8, cudaMemcpyDeviceToHost,
@@ -592,6 +592,7 @@ htrdr_gpu_server::loop_wave()
       && cuda_ok(cudaEventRecord(w_ev[b], io), "event");
     rb_k[b] = k;
     rb_epoch[b] = epoch;
+    rb_turn[b] = pool.turn;
     inflight[b] = ok;
     ++k;
     ++rounds;
@@ -641,43 +642,28 @@ htrdr_gpu_server::loop_wave()
       ++epoch;
     }
 
-    /* keep about one pool of realisations queued */
+    /* keep the queue filled */
     bool unqueued = false;
     for(SReq* r : active) unqueued |= r->state == 1 && r->next < r->total;
     const uint64_t queued = w_appended > dev_next ? w_appended - dev_next : 0;
-    if(unqueued && queued < wave_P) {
+    if(unqueued && queued < queue_depth) {
       const uint64_t before = w_appended;
-      if(!wave_append(active, wave_P - queued, k)) { failed_gpu = true; continue; }
-      if(w_appended > before) {
-        if(!cuda_ok(wave_serve_revive(wave, io), "revive")) { failed_gpu = true; continue; }
-        w_pool_live = true;
-      }
+      if(!wave_append(active, queue_depth - queued, k)) { failed_gpu = true; continue; }
+      if(w_appended > before) w_pool_live = true;
     }
 
-    if(w_pool_live) { /* one chunk, then the read-back of the previous launch */
+    if(w_pool_live) { /* one launch, then the read-back of the previous one */
       const int b = (int)(k & 1);
       if(inflight[b] && !process(b)) { failed_gpu = true; continue; }
-      if(!launch(b, false)) { failed_gpu = true; continue; }
+      if(!launch(b)) { failed_gpu = true; continue; }
       const int pb = b ^ 1;
-      if(inflight[pb] && !process(pb)) { failed_gpu = true; continue; }
+      const bool known = inflight[pb];
+      if(known && !process(pb)) { failed_gpu = true; continue; }
       retire(false);
-      /* drained: nothing queued, nothing left to queue, few live paths */
+      /* drained: nothing queued, nothing left to queue, no live path */
       bool more = false;
       for(SReq* r : active) more |= r->state == 1 && r->next < r->total;
-      if(dev_next >= w_appended && !more && !waiting) {
-        if(dev_live == 0) {
-          w_pool_live = false;
-        } else if(dev_live < wave_tail) { /* the tail: finish in the megakernel */
-          const int nb = (int)(k & 1);
-          if(inflight[nb] && !process(nb)) { failed_gpu = true; continue; }
-          if(!launch(nb, true)) { failed_gpu = true; continue; }
-          bool okp = true;
-          for(int i = 0; i < 2; ++i)
-            if(inflight[i]) okp = process(i) && okp;
-          if(!okp) { failed_gpu = true; continue; }
-          w_pool_live = false;
-        }
-      }
+      if(known && dev_next >= w_appended && !more && !waiting && dev_live == 0) w_pool_live = false;
       continue;
     }
 
@@ -716,7 +702,7 @@ try {
   /* smallest round: the configured first size, else two waves of resident threads */
   s->min_round = cfg->round_realisations
     ? (double)cfg->round_realisations
-    : 2.0 * (double)persistent_capacity(cfg->tuning.block_size, cfg->tuning.blocks_per_sm, cfg->device);
+    : 2.0 * (double)step_capacity(cfg->tuning.block_size, cfg->tuning.blocks_per_sm, cfg->device);
   s->round_real = s->min_round;
   bool ok = cuda_ok(cudaStreamCreateWithFlags(&s->io, cudaStreamNonBlocking), "stream");
   for(Slot& sl : s->slots)

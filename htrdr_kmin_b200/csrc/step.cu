@@ -1,0 +1,319 @@
+/* Kernels and launchers of the step loop (step.cuh) over the work queue: one
+ * launch that renders all queued realisations (the persistent and wavefront
+ * engines of the one-shot calls, graph batches and serving rounds), and the
+ * serving pool, whose launches end after a set time with the live paths
+ * saved, so that newly admitted requests join them in the next one. */
+#include "step.cuh"
+
+#include <algorithm>
+
+namespace hg {
+
+namespace {
+
+constexpr uint32_t kPathV4 = (uint32_t)((sizeof(Path) + 15) / 16);
+constexpr uint32_t kTraceV4 = (uint32_t)(sizeof(PathTrace) / 16);
+static_assert(sizeof(PathTrace) % 16 == 0, "the trace part is whole vectors");
+
+/* A saved path: kPathV4 consecutive 16-byte vectors */
+__device__ __forceinline__ void
+load_path(PathTrace& p, PathEvent& e, const uint4* v)
+{
+  uint4 t[kTraceV4], u[kPathV4 - kTraceV4];
+#pragma unroll
+  for(uint32_t i = 0; i < kTraceV4; ++i) t[i] = v[i];
+#pragma unroll
+  for(uint32_t i = kTraceV4; i < kPathV4; ++i) u[i - kTraceV4] = v[i];
+  memcpy(&p, t, sizeof(PathTrace));
+  memcpy(&e, u, sizeof(PathEvent));
+}
+
+__device__ __forceinline__ void
+save_path(const PathTrace& p, const PathEvent& e, uint4* v)
+{
+  uint4 t[kTraceV4], u[kPathV4 - kTraceV4];
+  u[kPathV4 - kTraceV4 - 1] = make_uint4(0, 0, 0, 0);
+  memcpy(t, &p, sizeof(PathTrace));
+  memcpy(u, &e, sizeof(PathEvent));
+#pragma unroll
+  for(uint32_t i = 0; i < kTraceV4; ++i) v[i] = t[i];
+#pragma unroll
+  for(uint32_t i = kTraceV4; i < kPathV4; ++i) v[i] = u[i - kTraceV4];
+}
+
+/* The work queue, and before it the paths a pool saved */
+template <bool Pool>
+struct QueueWork {
+  const DScene* scenes;
+  PTables T;
+  StepSums* sums;
+  /* Pool: saved paths read and written, their counters, the end of the launch */
+  const uint4* in;
+  uint4* out;
+  StepCtl* ctl;
+  uint32_t n_in, turn;
+  unsigned long long until;
+  bool saved_left;
+
+  __device__ __forceinline__ const DRequest& request(const PathEvent& e) const { return T.reqs[e.ri]; }
+
+  __device__ __forceinline__ bool stop()
+  {
+    if(!Pool) return false;
+    return __shfl_sync(HG_FULL, (int)(gtimer() >= until), 0) != 0;
+  }
+
+  __device__ __forceinline__ bool take(bool want, PathTrace& p, PathEvent& e)
+  {
+    const unsigned lane = threadIdx.x & 31u;
+    if(Pool && __any_sync(HG_FULL, saved_left)) {
+      const unsigned m = __ballot_sync(HG_FULL, want && saved_left);
+      if(m) {
+        const unsigned leader = __ffs(m) - 1;
+        uint32_t i0 = 0;
+        if(lane == leader) i0 = atomicAdd(&ctl->fetch, (uint32_t)__popc(m));
+        i0 = __shfl_sync(HG_FULL, i0, leader);
+        if(m & (1u << lane)) {
+          const uint32_t i = i0 + __popc(m & ((1u << lane) - 1u));
+          if(i < n_in) {
+            load_path(p, e, in + (size_t)i * kPathV4);
+            p.t0 = gtimer() - p.t0; /* saved: busy time so far */
+            want = false;
+          } else {
+            saved_left = false;
+          }
+        }
+      }
+    }
+    const unsigned m = __ballot_sync(HG_FULL, want);
+    if(!m) return true;
+    const unsigned leader = __ffs(m) - 1;
+    unsigned long long g0 = 0;
+    unsigned got = 0;
+    if(lane == leader) g0 = queue_take(T, (unsigned)__popc(m), &got);
+    g0 = __shfl_sync(HG_FULL, g0, leader);
+    got = __shfl_sync(HG_FULL, got, leader);
+    if(!want) return true;
+    const unsigned rank = __popc(m & ((1u << lane) - 1u));
+    if(rank >= got) return false;
+    path_assign(p, e.ri, T, g0 + rank);
+    return true;
+  }
+
+  __device__ __forceinline__ void done(PathTrace& p, PathEvent& e)
+  {
+    accumulate_b(p, e.weight, T.reqs[e.ri]);
+    count_grid(T.cnt, p);
+    sums->add(p);
+  }
+
+  /* The warp's paths to the pool, and the saved ones that no lane took */
+  __device__ __forceinline__ void save(PathTrace& p, PathEvent& e)
+  {
+    if(!Pool) return;
+    const unsigned lane = threadIdx.x & 31u;
+    bool keep = p.state != ST_IDLE;
+    for(;;) {
+      const unsigned m = __ballot_sync(HG_FULL, keep);
+      uint32_t o = 0;
+      if(lane == 0 && m) o = atomicAdd(&ctl->n[turn ^ 1u], (uint32_t)__popc(m));
+      o = __shfl_sync(HG_FULL, o, 0);
+      if(keep) {
+        p.t0 = gtimer() - p.t0;
+        save_path(p, e, out + (size_t)(o + __popc(m & ((1u << lane) - 1u))) * kPathV4);
+      }
+      uint32_t i0 = 0;
+      if(lane == 0) i0 = atomicAdd(&ctl->fetch, 32u);
+      i0 = __shfl_sync(HG_FULL, i0, 0);
+      if(i0 >= n_in) return;
+      keep = i0 + lane < n_in;
+      if(keep) {
+        load_path(p, e, in + (size_t)(i0 + lane) * kPathV4);
+        p.t0 = gtimer() - p.t0;
+      }
+    }
+  }
+};
+
+/* Paths a lane may hold: few ones are spread over all warps, as a warp with a
+ * single path takes its bounces fastest */
+__device__ __forceinline__ bool
+lane_unused(const PTables& T, uint32_t saved)
+{
+  const unsigned long long next = *(volatile unsigned long long*)T.next;
+  const unsigned long long left = saved + (T.total > next ? T.total - next : 0ull);
+  const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
+  return (threadIdx.x & 31u) >= (left + warps - 1) / warps;
+}
+
+template <unsigned V, bool Pool>
+__device__ __forceinline__ void
+step_block(PTables& T, const StepPool& P, int tables_in_smem)
+{
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ StepSums sums;
+  const bool unused = lane_unused(T, Pool ? P.ctl->n[P.turn] : 0u);
+  if(threadIdx.x == 0) sums = StepSums{0, 0, 0, 0, 0};
+  if(tables_in_smem) tables_to_smem(T, smem + step_event_bytes(blockDim.x));
+  __syncthreads();
+  QueueWork<Pool> work;
+  work.T = T;
+  work.scenes = T.scenes;
+  work.sums = &sums;
+  if(Pool) {
+    work.in = P.paths[P.turn];
+    work.out = P.paths[P.turn ^ 1u];
+    work.ctl = P.ctl;
+    work.turn = P.turn;
+    work.n_in = P.ctl->n[P.turn];
+    work.until = gtimer() + P.ns;
+    work.saved_left = work.n_in != 0;
+  }
+  PathTrace p;
+  const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
+  step_loop<V>(work, p, ((PathEvent*)smem)[threadIdx.x], unused || (Pool && id >= P.lanes));
+  __syncthreads();
+  if(threadIdx.x == 0) {
+    Counters* c = (Counters*)T.cnt;
+    atomicAdd(&c->seg, sums.seg);
+    atomicAdd(&c->node, sums.node);
+    atomicAdd(&c->tc, sums.tc);
+    atomicAdd(&c->real, sums.real);
+    atomicAdd(&c->fail, sums.fail);
+  }
+}
+
+}  // namespace
+
+template <unsigned V>
+__global__ void __maxnreg__(step_registers(V))
+k_step(PTables T, int tables_in_smem)
+{
+  step_block<V, false>(T, StepPool{}, tables_in_smem);
+}
+
+template <unsigned V>
+__global__ void __maxnreg__(step_registers(V))
+k_step_pool(PTables T, StepPool P, int tables_in_smem)
+{
+  step_block<V, true>(T, P, tables_in_smem);
+}
+
+/* After a launch of a pool: the paths it read are free, and the queue's head
+ * goes back to the queued total, so that work appended later starts there */
+__global__ void
+k_step_turn(PTables T, StepCtl* ctl, uint32_t read)
+{
+  ctl->n[read] = 0;
+  ctl->fetch = 0;
+  queue_clamp(T);
+}
+
+namespace {
+
+using StepFn = void (*)(PTables, int);
+using StepPoolFn = void (*)(PTables, StepPool, int);
+StepFn
+step_fn(uint32_t v)
+{
+  HG_PICK_VARIANT(v, k_step)
+}
+StepPoolFn
+step_pool_fn(uint32_t v)
+{
+  HG_PICK_VARIANT(v, k_step_pool)
+}
+
+/* Grid of a kernel of `threads' threads a block that fills the device */
+template <class Fn>
+cudaError_t
+step_shape(Fn kern, const PTables& T, uint32_t threads, uint32_t blocks_per_sm, int device, size_t* smem,
+           int* in_smem, unsigned* grid)
+{
+  const size_t tables = ((T.nscenes * sizeof(DScene) + 15) & ~(size_t)15) + T.nreqs * sizeof(DRequest);
+  *in_smem = tables <= 96 * 1024;
+  *smem = step_event_bytes(threads) + (*in_smem ? tables : 0);
+  if(*smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem);
+    if(e != cudaSuccess) return e;
+  }
+  int nsm = 0, per_sm = 0;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (int)threads, *smem);
+  if(blocks_per_sm) per_sm = std::min(per_sm, (int)blocks_per_sm);
+  *grid = (unsigned)(nsm * std::max(per_sm, 1));
+  return cudaSuccess;
+}
+
+}  // namespace
+
+cudaError_t
+launch_step(const PTables& T, uint32_t block_size, uint32_t blocks_per_sm, int device, cudaStream_t st)
+{
+  if(!T.total) return cudaSuccess;
+  auto kern = step_fn(T.variant);
+  size_t smem;
+  int in_smem;
+  unsigned grid;
+  const cudaError_t e = step_shape(kern, T, block_size, blocks_per_sm, device, &smem, &in_smem, &grid);
+  if(e != cudaSuccess) return e;
+  kern<<<grid, block_size, smem, st>>>(T, in_smem);
+  note_launches(1);
+  return cudaGetLastError();
+}
+
+uint64_t
+step_capacity(uint32_t block_size, uint32_t blocks_per_sm, int device)
+{
+  PTables T{};
+  size_t smem;
+  int in_smem;
+  unsigned grid;
+  if(step_shape(k_step<HV_ALL>, T, block_size, blocks_per_sm, device, &smem, &in_smem, &grid)) return 0;
+  return (uint64_t)grid * block_size;
+}
+
+/* ---- serving pool ---- */
+
+/* Threads a block of the pool's launches, and lanes an SM at most (any variant
+ * takes 64 registers or more) */
+constexpr uint32_t kPoolThreads = 128, kPoolLanesPerSm = 1024;
+
+bool
+step_pool_create(StepBufs& B, uint32_t lanes, int device, cudaStream_t st)
+{
+  /* room for the lanes of any variant: a launch carries over what the one
+   * before it saved */
+  int nsm = 0;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
+  const size_t most = (size_t)nsm * kPoolLanesPerSm;
+  B.lanes = lanes ? (uint32_t)std::min<size_t>(lanes, most) : (uint32_t)most;
+  for(int i = 0; i < 2; ++i)
+    if(!B.paths[i].alloc((size_t)B.lanes * kPathV4 * 16)) return false;
+  return B.ctl.alloc(sizeof(StepCtl)) && cuda_ok(cudaMemsetAsync(B.ctl.ptr, 0, sizeof(StepCtl), st), "memset");
+}
+
+cudaError_t
+step_pool_launch(const PTables& T, StepBufs& B, uint64_t ns, uint32_t blocks_per_sm, int device, cudaStream_t st)
+{
+  StepPool P;
+  P.paths[0] = (uint4*)B.paths[0].ptr;
+  P.paths[1] = (uint4*)B.paths[1].ptr;
+  P.ctl = (StepCtl*)B.ctl.ptr;
+  P.turn = B.turn;
+  P.lanes = B.lanes;
+  P.ns = ns;
+  auto kern = step_pool_fn(T.variant);
+  size_t smem;
+  int in_smem;
+  unsigned grid;
+  const cudaError_t e = step_shape(kern, T, kPoolThreads, blocks_per_sm, device, &smem, &in_smem, &grid);
+  if(e != cudaSuccess) return e;
+  kern<<<grid, kPoolThreads, smem, st>>>(T, P, in_smem);
+  k_step_turn<<<1, 1, 0, st>>>(T, P.ctl, B.turn);
+  B.turn ^= 1u;
+  note_launches(2);
+  return cudaGetLastError();
+}
+
+}  // namespace hg

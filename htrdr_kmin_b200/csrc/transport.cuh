@@ -475,10 +475,9 @@ struct Counters {
   unsigned long long seg, node, tc, real, fail, grid;
 };
 
-/* Trace part of a path: everything trace_step reads or writes, and the walk
- * fields the wavefront's trace stage touches when it runs a LW scattering
- * itself.  It comes first so that the trace stage moves only this prefix of a
- * stored path. */
+/* Trace part of a path: everything trace_step reads or writes, and what a LW
+ * scattering in the medium does.  The step loop keeps it in registers and the
+ * event part in shared memory. */
 struct PathTrace {
   Rng rng;
   uint32_t c_grid;      /* local counter of leaf-grid bytes read (the word before
@@ -782,8 +781,7 @@ region_leave(PathTrace& p)
 /* SW walk after a free path that ended by a collision in the medium: the
  * absorption transmissivity along that free path, from its origin to the
  * collision site (..._sw.c:385-398).  It reads and writes only the trace
- * part of the path, so the wavefront's trace stage runs it in place of an
- * event-stage visit.  Returns the collision site (pos_next). */
+ * part of the path.  Returns the collision site (pos_next). */
 __device__ __forceinline__ float3
 sw_scat_volume(PathTrace& p, TraceArgs& q)
 {
@@ -1333,9 +1331,8 @@ lw_plane_ground(const DScene& S)
  * steps ST_LW_END and ST_LW_WALK take there.  It reads and writes the trace
  * part of the path only (the plane's hit record, set at the walk's first
  * ground query, stays the same); the origin and direction of the free path it
- * asks for are the walk's new position and direction, which the wavefront's
- * trace stage stores into p.pos / p.dir: the stage runs it without an
- * event-stage visit.  The caller checks that
+ * asks for are the walk's new position and direction, which the step loop
+ * stores into e.pos / e.dir: it goes on without path_event().  The caller checks that
  * the bounce limit is not reached. */
 __device__ __forceinline__ void
 lw_scatter_plane(PathTrace& p, const DScene& S, TraceArgs& q)
@@ -1479,9 +1476,6 @@ path_event(PathTrace& p, PathEvent& e, const DScene& S, const DRequest& R)
       }
 
       case ST_LW_END: if constexpr(!(V & HV_LW)) { path_variant_miss(p); break; } else {
-        /* the free path just traced started at p.tr.o along p.tr.d (the
-         * walk's position and direction, which the trace stage may have
-         * moved past e.pos / e.dir) */
         const bool svx = p.tr.hit != 0;
         if(p.gdist < 0.f && !svx) { e.w = 0.0; p.state = ST_RAD_END; break; }
         const float tdst = svx ? p.tr.tcur : p.gdist;

@@ -183,9 +183,9 @@ HTRDR_GPU_API uint32_t htrdr_gpu_scene_tree_depth(const struct htrdr_gpu_scene* 
  * structs (src/atmosphere/htrdr_atmosphere_c.h:46-76).
  *
  * Three engines compute the same per-realisation weights (only the FP64
- * summation order of a pixel differs): the persistent megakernel with its
- * work queue, the wavefront engine (event and trace stage kernels over a
- * pool of path slots in HBM, same work queue) and the plain
+ * summation order of a pixel differs): the step loop over a work queue
+ * (_PERSISTENT and _WAVEFRONT, which differ in serving only), the
+ * block-sorted kernel and the plain
  * one-thread-per-realisation kernel. ---- */
 enum htrdr_gpu_engine {
   HTRDR_GPU_ENGINE_PERSISTENT = 0,
@@ -319,18 +319,15 @@ struct htrdr_gpu_batch_item {
   void* buffer; /* host */
 };
 struct htrdr_gpu_tuning {
-  uint32_t block_size;    /* threads per block of the persistent kernel (wavefront: of its
-                           * trace stage) */
-  uint32_t queue_chunk;   /* realisations taken from the work queue at once (persistent) */
-  uint32_t regroup_period;/* voxel steps between two regroupings of a warp's lanes (events and
-                           * new realisations run together; 0 or 1: every step) (persistent, and
-                           * the megakernel that finishes a wavefront run) */
+  uint32_t block_size;    /* threads per block */
+  uint32_t queue_chunk;   /* not used (the step loop's lanes take work as they run dry); >= 1 */
+  uint32_t regroup_period;/* sorted: voxel steps of a trace per regrouping of the block's paths */
   uint32_t blocks_per_sm; /* resident blocks per SM (0: occupancy maximum) */
   uint32_t engine;        /* HTRDR_GPU_ENGINE_PERSISTENT, _WAVEFRONT or _SORTED */
-  uint32_t wave_slots;    /* wavefront: paths in flight (0: 2^21, at most the realisations) */
-  uint32_t trace_budget;  /* wavefront: voxel steps of a trace per trace-stage visit (0: 256) */
-  uint32_t wave_tail;     /* wavefront: live paths below which the remaining ones finish in one
-                           * megakernel launch (0: four waves of its resident threads) */
+  uint32_t wave_slots;    /* wavefront serving: paths in flight and realisations queued (0: all
+                           * resident lanes, and 2^21) */
+  uint32_t trace_budget;  /* not used */
+  uint32_t wave_tail;     /* not used */
 };
 /* Renders every item (each one htrdr_draw_map call of the reference) in one
  * persistent kernel; item buffers are host memory.  tuning == NULL: the
@@ -352,22 +349,18 @@ htrdr_gpu_draw_maps_batched_accum_device(struct htrdr_gpu_batch_item* items, siz
                                          const struct htrdr_gpu_tuning* tuning,
                                          struct htrdr_gpu_stats* stats);
 HTRDR_GPU_API void htrdr_gpu_default_tuning(struct htrdr_gpu_tuning* tuning);
-/* Default tuning of a request mode: the wavefront engine (trace-stage blocks
- * of 256, 256 voxel steps per visit, 2^21 path slots), its tail megakernel
- * taking over below 25 000 live paths for SW, 100 000 for CIE and LW. */
+/* Default tuning of a request mode: the step loop in blocks of 256. */
 HTRDR_GPU_API void htrdr_gpu_mode_tuning(int mode, struct htrdr_gpu_tuning* tuning);
-/* Autotuner: times the candidate tunings (persistent: block size, queue
- * chunk, regroup period; wavefront: tail threshold, regroup period) on
- * `items' (device buffers) and returns the fastest; the rendered values do
- * not depend on the tuning. */
+/* Autotuner: times the step loop's candidate block sizes on `items' (device
+ * buffers) and returns the fastest; the rendered values do not depend on the
+ * tuning. */
 HTRDR_GPU_API htrdr_gpu_res_T
 htrdr_gpu_autotune(struct htrdr_gpu_batch_item* items, size_t n, struct htrdr_gpu_tuning* best,
                    double* best_ms);
 
 /* Reusable batch (item buffers are device memory): the launch sequence is
  * captured once in a CUDA graph; every run replays it.  The tuning's engine
- * must be the persistent one (the wavefront's iteration count is decided on
- * the host while it runs): BAD_ARG otherwise. */
+ * must be a persistent one: BAD_ARG for _WAVEFRONT. */
 struct htrdr_gpu_batch;
 HTRDR_GPU_API htrdr_gpu_res_T
 htrdr_gpu_batch_create(const struct htrdr_gpu_batch_item* items, size_t n,
@@ -382,7 +375,7 @@ HTRDR_GPU_API void htrdr_gpu_batch_release(struct htrdr_gpu_batch* batch);
  * accumulators + output staging) fits in the HBM budget, keeps their
  * accumulators resident, and feeds a fair share of every admitted request's
  * remaining realisations to the engine: rounds of the persistent kernel, or
- * the wavefront's work queue, whose path slots take the realisations of newly
+ * a pool of paths in flight, whose lanes take the realisations of newly
  * admitted requests as soon as their paths end.  Requests that arrive while
  * others render join the running work.  A request completes when all its
  * realisations are accumulated: its map is copied to its host buffer. */
@@ -391,10 +384,9 @@ struct htrdr_gpu_server_config {
   size_t hbm_budget_bytes;       /* admission budget for per-request device memory */
   double round_target_ms;        /* rounds hold ~ this much work at the observed throughput */
   uint64_t round_realisations;   /* smallest round (0: two waves of the kernel's resident threads) */
-  struct htrdr_gpu_tuning tuning;  /* persistent: rounds of the megakernel on three streams;
-                                    * wavefront: one pool of path slots fed by a growing
-                                    * queue (wave_slots paths, held for the server's
-                                    * lifetime) */
+  struct htrdr_gpu_tuning tuning;  /* persistent: rounds on three streams; wavefront: one pool
+                                    * of paths, resumed launch after launch, fed by a
+                                    * growing queue */
 };
 struct htrdr_gpu_server_stats {
   uint64_t submitted, completed, failed, rounds, realisations;
@@ -421,7 +413,7 @@ htrdr_gpu_server_wait(struct htrdr_gpu_server* server, uint64_t ticket, double t
                       htrdr_gpu_res_T* result);
 HTRDR_GPU_API htrdr_gpu_res_T
 htrdr_gpu_server_stats(struct htrdr_gpu_server* server, struct htrdr_gpu_server_stats* stats);
-/* Launches of the request loop (persistent rounds or wavefront chunks,
+/* Launches of the request loop (rounds, or launches of the pool,
  * numbered from 0 in launch order) that carried a request: `first', the
  * first with some of its realisations queued, and `last', the last before
  * all of them were known done.  Two requests whose ranges intersect had work

@@ -780,7 +780,7 @@ def measure(args, api, su: "Setup", desc: str, tuning, tuning_src: str, rank: in
     peak, peak_kind = peaks()
     achieved = alg_bytes / (kms * 1e-3) / 1e9
     kernel = "k_sorted" if tuning.engine == api.ENGINE_SORTED else "k_step"
-    traffic, traffic_src = traffic_per_launch(traffic_key or ("wavefront" if kernel == "k_step" else kernel), alg_bytes)
+    traffic, traffic_src = traffic_per_launch(traffic_key or kernel, alg_bytes)
     out_bytes = sum(d.numel() for d in su.dev)
     line = {
         "value": world * reals / (step_ms * 1e-3) / 1e6, "ms_per_step": step_ms,
@@ -874,7 +874,7 @@ def main():
         return
     tuning, src = pick_tuning(args, api, su, args.workload)
     fields, gpu_maps, _ = measure(args, api, su, desc, tuning, src, rank, world, dist,
-                                  traffic_key="wavefront_lw" if (args.workload == "lw_flux"
+                                  traffic_key="k_step_lw" if (args.workload == "lw_flux"
                                                                  and tuning.engine != api.ENGINE_SORTED) else "")
 
     line = {"metric": METRIC, "value": fields.pop("value"), "unit": UNIT, "n_gpus": world,
@@ -918,7 +918,7 @@ def main():
         t2, src2 = pick_tuning(args, api, su2, "lw_flux") if not args.tuning else (
             api.mode_tuning(S.MODE_FLUX_LW), "mode default")
         f2, _, _ = measure(args, api, su2, desc2, t2, src2, rank, world, dist, clocks=False,
-                           traffic_key="wavefront_lw" if t2.engine != api.ENGINE_SORTED else "")
+                           traffic_key="k_step_lw" if t2.engine != api.ENGINE_SORTED else "")
         line["lw_flux"] = {k: f2[k] for k in ("value", "ms_per_step", "e2e", "plain_gpu",
                                               "batched_vs_plain", "roofline", "segments_per_s")}
         line["lw_flux"]["unit"] = UNIT

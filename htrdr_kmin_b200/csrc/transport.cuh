@@ -378,6 +378,15 @@ ground_query(const DScene& S, float3 o, float3 d, float r1, bool prev, uint32_t 
     *ng = make_float3(0.f, 0.f, 1.f);
     return ground_trace(S, o, d, 0.f, r1, prev);
   }
+  /* a ray that leaves the height range of the repeated mesh (most rays of a
+   * cloud that go up): no copy of it can be met, as g_trace() would find with
+   * two FP64 divisions */
+  if(S.g_repeat && (d.z > 0.f ? (double)o.z > S.g_upper[2] : d.z < 0.f && (double)o.z < S.g_lower[2])) {
+    *prim = HG_NO_PRIM;
+    *edge = false;
+    *ng = make_float3(0.f, 0.f, 0.f);
+    return -1.f;
+  }
   const GHit h = g_trace(S, o, d, 0.f, r1, prev ? prev_prim : HG_NO_PRIM, prev && prev_edge);
   *prim = h.prim;
   *edge = h.prim != HG_NO_PRIM && g_on_edge(h.u, h.v);

@@ -89,14 +89,14 @@ single_tables_bytes()
 }
 
 cudaError_t
-launch_workqueue(const PTables& T0, const htrdr_gpu_tuning& tun, int device, cudaStream_t st)
+launch_workqueue(const PTables& T0, const htrdr_gpu_tuning& tun, int device, cudaStream_t st, bool may_keep)
 {
   PTables T = T0;
   T.chunk = tun.queue_chunk;
   T.regroup_period = tun.regroup_period;
   return tun.engine == HTRDR_GPU_ENGINE_SORTED
     ? launch_sorted(T, tun.block_size, tun.blocks_per_sm, device, st)
-    : launch_step(T, tun.block_size, tun.blocks_per_sm, device, st);
+    : launch_step(T, tun.block_size, tun.blocks_per_sm, device, st, may_keep);
 }
 
 cudaError_t
@@ -125,7 +125,7 @@ launch_workqueue_single(const DScene& S, const DRequest& R, void* tables, void* 
   T.total = h.offsets[1];
   T.cnt = cnt;
   T.next = (unsigned long long*)((char*)cnt + 64);
-  return launch_workqueue(T, tun, device, st);
+  return launch_workqueue(T, tun, device, st, true);
 }
 
 /* Device buffers of a plan: tables, accumulators, counters, output staging */
@@ -277,7 +277,7 @@ plan_enqueue(Plan& P, const htrdr_gpu_batch_item* items, size_t n, const htrdr_g
    * the replays */
   const unsigned evf = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
   if(ok && k0) ok = cuda_ok(cudaEventRecordWithFlags(k0, st, evf), "event");
-  if(ok) ok = cuda_ok(launch_workqueue(P.T, tun, P.device, st), "k_step");
+  if(ok) ok = cuda_ok(launch_workqueue(P.T, tun, P.device, st, !capturing), "k_step");
   if(ok && k1) ok = cuda_ok(cudaEventRecordWithFlags(k1, st, evf), "event");
   for(size_t i = 0; ok && !P.accum_out && i < n; ++i) {
     char* dout = host_out ? (char*)P.B->d_out.ptr + P.out_off[i] : (char*)items[i].buffer;

@@ -198,11 +198,22 @@ radiance_impl(htrdr_gpu_scene* scn, int lw, size_t n, const double* pos, const d
   }
   if(!n) return HTRDR_GPU_RES_OK;
   if(!cuda_ok(cudaSetDevice(scn->device), "cudaSetDevice")) return HTRDR_GPU_RES_BAD_OP;
-  /* one allocation for the rays, the radiances and the counter: each of six
-   * buffers cost its allocation and, at its release, a device-wide wait */
-  DevBuf buf;
-  if(!buf.alloc(n * (8 * 8 + 2 * 4) + 16)) return HTRDR_GPU_RES_MEM_ERR;
-  double* d = (double*)buf.ptr;
+  /* One allocation for the rays, the radiances and the counter, kept by the
+   * scene for its next call: each of six buffers cost its allocation and, at
+   * its release, a device-wide wait of up to 20 ms.  A call that finds it in
+   * use by another thread has its own. */
+  constexpr size_t kKeepRays = (size_t)256 << 20;
+  const size_t bytes = n * (8 * 8 + 2 * 4) + 16;
+  std::unique_ptr<DevBuf> buf;
+  {
+    std::lock_guard<std::mutex> lock(scn->mtx);
+    buf = std::move(scn->rays);
+  }
+  if(!buf || buf->bytes < bytes) {
+    buf = std::make_unique<DevBuf>();
+    if(!buf->alloc(bytes)) return HTRDR_GPU_RES_MEM_ERR;
+  }
+  double* d = (double*)buf->ptr;
   RayArgs a;
   a.lw = lw;
   a.mask = mask;
@@ -225,7 +236,12 @@ radiance_impl(htrdr_gpu_scene* scn, int lw, size_t n, const double* pos, const d
                && cuda_ok(launch_radiance(scn->d, a, scn->device, st), "k_radiance")
                && cuda_ok(cudaMemcpyAsync(out, a.out, 8 * n, cudaMemcpyDeviceToHost, st), "D2H");
   /* also after an error: the copies in flight read the caller's arrays */
-  return cuda_ok(cudaStreamSynchronize(st), "sync") && ok ? HTRDR_GPU_RES_OK : HTRDR_GPU_RES_UNKNOWN_ERR;
+  const bool synced = cuda_ok(cudaStreamSynchronize(st), "sync");
+  if(bytes <= kKeepRays) {
+    std::lock_guard<std::mutex> lock(scn->mtx);
+    if(!scn->rays) scn->rays = std::move(buf);
+  }
+  return synced && ok ? HTRDR_GPU_RES_OK : HTRDR_GPU_RES_UNKNOWN_ERR;
 }
 
 extern "C" HTRDR_GPU_API htrdr_gpu_res_T

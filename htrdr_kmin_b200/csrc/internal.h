@@ -79,6 +79,9 @@ struct htrdr_gpu_scene {
   /* Wavelength samplers keyed by (cie, range0, range1, Tref) */
   std::map<std::tuple<int, double, double, double>, std::unique_ptr<hg::Sampler>> samplers;
   std::mutex mtx;
+  /* rays and radiances of the last radiance call (at most kKeepRays bytes; no
+   * entry while a call uses it) */
+  std::unique_ptr<hg::DevBuf> rays;
   cudaStream_t stream = nullptr;
   /* engine of draw_map on this scene (enum htrdr_gpu_engine; engine_set == 0:
    * the mode's default) and the tuning of the work-queue engines
@@ -207,9 +210,11 @@ bool valid_tuning(const htrdr_gpu_tuning& t);
  * zeroed before the launch. */
 size_t single_tables_bytes();
 
-/* Step loop (step.cu): all queued realisations of T in one launch */
+/* Step loop (step.cu): all queued realisations of T.  may_keep: the calling
+ * thread's buffer for the last paths may be used (not by launches that overlap
+ * others of the thread, nor by captured ones) */
 cudaError_t launch_step(const PTables& T, uint32_t block_size, uint32_t blocks_per_sm, int device,
-                        cudaStream_t st);
+                        cudaStream_t st, bool may_keep);
 /* Threads that launch keeps resident on the device */
 uint64_t step_capacity(uint32_t block_size, uint32_t blocks_per_sm, int device);
 
@@ -235,7 +240,8 @@ bool step_pool_create(StepBufs& B, uint32_t lanes, int device, cudaStream_t st);
 cudaError_t step_pool_launch(const PTables& T, StepBufs& B, uint64_t ns, uint32_t blocks_per_sm, int device,
                              cudaStream_t st);
 /* One launch of a work-queue engine over T (tun.engine) */
-cudaError_t launch_workqueue(const PTables& T, const htrdr_gpu_tuning& tun, int device, cudaStream_t st);
+cudaError_t launch_workqueue(const PTables& T, const htrdr_gpu_tuning& tun, int device, cudaStream_t st,
+                             bool may_keep);
 /* The same for one request; the tables are staged in `tables' */
 cudaError_t launch_workqueue_single(const DScene& S, const DRequest& R, void* tables, void* cnt,
                                     const htrdr_gpu_tuning& tun, int device, cudaStream_t st);

@@ -231,7 +231,7 @@ htrdr_gpu_server::launch_round(Slot& s, const std::vector<SReq*>& act)
   T.chunk = cfg.tuning.queue_chunk;
   T.regroup_period = cfg.tuning.regroup_period;
   ok = ok && cuda_ok(cudaEventRecord(s.e0, s.st), "event")
-          && cuda_ok(launch_workqueue(T, cfg.tuning, cfg.device, s.st), "k_step")
+          && cuda_ok(launch_workqueue(T, cfg.tuning, cfg.device, s.st, false), "k_step")
           && cuda_ok(cudaEventRecord(s.e1, s.st), "event");
   realisations += T.total;
   s.busy = true;

@@ -3,9 +3,11 @@
  * engines of the one-shot calls, graph batches and serving rounds), and the
  * serving pool, whose launches end after a set time with the live paths
  * saved, so that newly admitted requests join them in the next one. */
-#include "step.cuh"
+#include "pair.cuh"
 
 #include <algorithm>
+#include <map>
+#include <memory>
 
 namespace hg {
 
@@ -41,9 +43,22 @@ save_path(const PathTrace& p, const PathEvent& e, uint4* v)
   for(uint32_t i = kTraceV4; i < kPathV4; ++i) v[i] = u[i - kTraceV4];
 }
 
-/* The work queue, and before it the paths a pool saved */
-template <bool Pool>
+/* Where a launch's paths come from and go to: the queue alone; a pool, whose
+ * saved paths come before the queue and which saves the live ones when the
+ * launch's time is over; the queue, and the last paths saved for another
+ * launch when it has run dry (LAST_OUT) and taken up by that one (LAST_IN) */
+enum { WK_QUEUE = 0, WK_POOL, WK_LAST_OUT, WK_LAST_IN };
+
+/* Live paths of a warp that has found the queue dry at which it hands them
+ * over.  Measured (6 / 12 / 20 / 24 / 32, and none handed over): SW image of
+ * 131 000 realisations 13.0 / 12.7 / 12.0 / 12.0 / 12.5, 12.8 ms; flux map 29.0 /
+ * 27.7 / 26.6 / 26.8 / 26.9, 28.0; CIE image 16.4 / 16.2 / 14.6 / 15.0 / 15.1,
+ * 16.6; mesh image 33.2 / 31.2 / 30.1 / 30.6 / 29.7, 32.7. */
+constexpr uint32_t kLastPaths = 20;
+
+template <int Kind>
 struct QueueWork {
+  static constexpr bool kReads = Kind == WK_POOL || Kind == WK_LAST_IN;
   const DScene* scenes;
   PTables T;
   StepSums* sums;
@@ -53,20 +68,20 @@ struct QueueWork {
   StepCtl* ctl;
   uint32_t n_in, turn;
   unsigned long long until;
-  bool saved_left;
+  bool saved_left, dry;
 
   __device__ __forceinline__ const DRequest& request(const PathEvent& e) const { return T.reqs[e.ri]; }
 
-  __device__ __forceinline__ bool stop()
+  __device__ __forceinline__ bool stop(uint32_t live)
   {
-    if(!Pool) return false;
-    return __shfl_sync(HG_FULL, (int)(gtimer() >= until), 0) != 0;
+    if(Kind == WK_POOL) return __shfl_sync(HG_FULL, (int)(gtimer() >= until), 0) != 0;
+    return Kind == WK_LAST_OUT && live <= kLastPaths && __any_sync(HG_FULL, dry);
   }
 
   __device__ __forceinline__ bool take(bool want, PathTrace& p, PathEvent& e)
   {
     const unsigned lane = threadIdx.x & 31u;
-    if(Pool && __any_sync(HG_FULL, saved_left)) {
+    if(kReads && __any_sync(HG_FULL, saved_left)) {
       const unsigned m = __ballot_sync(HG_FULL, want && saved_left);
       if(m) {
         const unsigned leader = __ffs(m) - 1;
@@ -93,6 +108,7 @@ struct QueueWork {
     if(lane == leader) g0 = queue_take(T, (unsigned)__popc(m), &got);
     g0 = __shfl_sync(HG_FULL, g0, leader);
     got = __shfl_sync(HG_FULL, got, leader);
+    if(got < (unsigned)__popc(m)) dry = true;
     if(!want) return true;
     const unsigned rank = __popc(m & ((1u << lane) - 1u));
     if(rank >= got) return false;
@@ -110,7 +126,7 @@ struct QueueWork {
   /* The warp's paths to the pool, and the saved ones that no lane took */
   __device__ __forceinline__ void save(PathTrace& p, PathEvent& e)
   {
-    if(!Pool) return;
+    if(Kind != WK_POOL && Kind != WK_LAST_OUT) return;
     const unsigned lane = threadIdx.x & 31u;
     bool keep = p.state != ST_IDLE;
     for(;;) {
@@ -122,6 +138,7 @@ struct QueueWork {
         p.t0 = gtimer() - p.t0;
         save_path(p, e, out + (size_t)(o + __popc(m & ((1u << lane) - 1u))) * kPathV4);
       }
+      if(!kReads) return;
       uint32_t i0 = 0;
       if(lane == 0) i0 = atomicAdd(&ctl->fetch, 32u);
       i0 = __shfl_sync(HG_FULL, i0, 0);
@@ -135,52 +152,66 @@ struct QueueWork {
   }
 };
 
-/* Paths a lane may hold: few ones are spread over all warps, as a warp with a
- * single path takes its bounces fastest */
+/* Whether this lane stays empty: few paths are spread over all warps, as a
+ * warp with a single path takes its bounces fastest */
 __device__ __forceinline__ bool
-lane_unused(const PTables& T, uint32_t saved)
+lane_unused(const PTables& T, uint32_t saved, uint32_t warps_per_block)
 {
   const unsigned long long next = *(volatile unsigned long long*)T.next;
   const unsigned long long left = saved + (T.total > next ? T.total - next : 0ull);
-  const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
+  const unsigned long long warps = (unsigned long long)gridDim.x * warps_per_block;
   return (threadIdx.x & 31u) >= (left + warps - 1) / warps;
 }
 
-template <unsigned V, bool Pool>
+template <int Kind>
+__device__ __forceinline__ QueueWork<Kind>
+queue_work(const PTables& T, StepSums* sums, const StepPool& P)
+{
+  QueueWork<Kind> work;
+  work.T = T;
+  work.scenes = T.scenes;
+  work.sums = sums;
+  work.dry = false;
+  work.saved_left = false;
+  if(Kind != WK_QUEUE) {
+    work.in = P.paths[P.turn];
+    work.out = P.paths[P.turn ^ 1u];
+    work.ctl = P.ctl;
+    work.turn = P.turn;
+    work.n_in = work.kReads ? P.ctl->n[P.turn] : 0u;
+    work.until = gtimer() + P.ns;
+    work.saved_left = work.n_in != 0;
+  }
+  return work;
+}
+
+__device__ __forceinline__ void
+flush_sums(const PTables& T, const StepSums& sums)
+{
+  Counters* c = (Counters*)T.cnt;
+  atomicAdd(&c->seg, sums.seg);
+  atomicAdd(&c->node, sums.node);
+  atomicAdd(&c->tc, sums.tc);
+  atomicAdd(&c->real, sums.real);
+  atomicAdd(&c->fail, sums.fail);
+}
+
+template <unsigned V, int Kind>
 __device__ __forceinline__ void
 step_block(PTables& T, const StepPool& P, int tables_in_smem)
 {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ StepSums sums;
-  const bool unused = lane_unused(T, Pool ? P.ctl->n[P.turn] : 0u);
+  const bool unused = lane_unused(T, QueueWork<Kind>::kReads ? P.ctl->n[P.turn] : 0u, blockDim.x >> 5);
   if(threadIdx.x == 0) sums = StepSums{0, 0, 0, 0, 0};
   if(tables_in_smem) tables_to_smem(T, smem + step_event_bytes(blockDim.x));
   __syncthreads();
-  QueueWork<Pool> work;
-  work.T = T;
-  work.scenes = T.scenes;
-  work.sums = &sums;
-  if(Pool) {
-    work.in = P.paths[P.turn];
-    work.out = P.paths[P.turn ^ 1u];
-    work.ctl = P.ctl;
-    work.turn = P.turn;
-    work.n_in = P.ctl->n[P.turn];
-    work.until = gtimer() + P.ns;
-    work.saved_left = work.n_in != 0;
-  }
+  QueueWork<Kind> work = queue_work<Kind>(T, &sums, P);
   PathTrace p;
   const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
-  step_loop<V>(work, p, ((PathEvent*)smem)[threadIdx.x], unused || (Pool && id >= P.lanes));
+  step_loop<V>(work, p, ((PathEvent*)smem)[threadIdx.x], unused || (Kind == WK_POOL && id >= P.lanes));
   __syncthreads();
-  if(threadIdx.x == 0) {
-    Counters* c = (Counters*)T.cnt;
-    atomicAdd(&c->seg, sums.seg);
-    atomicAdd(&c->node, sums.node);
-    atomicAdd(&c->tc, sums.tc);
-    atomicAdd(&c->real, sums.real);
-    atomicAdd(&c->fail, sums.fail);
-  }
+  if(threadIdx.x == 0) flush_sums(T, sums);
 }
 
 }  // namespace
@@ -189,14 +220,47 @@ template <unsigned V>
 __global__ void __maxnreg__(step_registers(V))
 k_step(PTables T, int tables_in_smem)
 {
-  step_block<V, false>(T, StepPool{}, tables_in_smem);
+  step_block<V, WK_QUEUE>(T, StepPool{}, tables_in_smem);
 }
 
 template <unsigned V>
 __global__ void __maxnreg__(step_registers(V))
 k_step_pool(PTables T, StepPool P, int tables_in_smem)
 {
-  step_block<V, true>(T, P, tables_in_smem);
+  step_block<V, WK_POOL>(T, P, tables_in_smem);
+}
+
+/* All but the last paths of a run */
+template <unsigned V>
+__global__ void __maxnreg__(step_registers(V))
+k_step_most(PTables T, StepPool P, int tables_in_smem)
+{
+  step_block<V, WK_LAST_OUT>(T, P, tables_in_smem);
+}
+
+/* The last paths of a run, or a small run: two warps a path (pair.cuh) */
+template <unsigned V>
+__global__ void __launch_bounds__(64 * kPairs, 1)
+k_pair(PTables T, StepPool P, int tables_in_smem)
+{
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ StepSums sums;
+  __shared__ uint32_t live[kPairs];
+  const bool unused = lane_unused(T, P.ctl->n[P.turn], kPairs);
+  if(threadIdx.x == 0) sums = StepSums{0, 0, 0, 0, 0};
+  PairJob* jobs = (PairJob*)(smem + step_event_bytes(32 * kPairs));
+  if(tables_in_smem) tables_to_smem(T, smem + pair_bytes());
+  __syncthreads();
+  QueueWork<WK_LAST_IN> work = queue_work<WK_LAST_IN>(T, &sums, P);
+  const uint32_t pair = (threadIdx.x >> 5) % kPairs, slot = threadIdx.x % (32 * kPairs);
+  if(threadIdx.x < 32 * kPairs) {
+    PathTrace p;
+    pair_main<V>(work, p, ((PathEvent*)smem)[slot], jobs[slot], live[pair], (int)pair, unused);
+  } else {
+    pair_partner<V>(work, jobs[slot], live[pair], (int)pair);
+  }
+  __syncthreads();
+  if(threadIdx.x == 0) flush_sums(T, sums);
 }
 
 /* After a launch of a pool: the paths it read are free, and the queue's head
@@ -223,16 +287,37 @@ step_pool_fn(uint32_t v)
 {
   HG_PICK_VARIANT(v, k_step_pool)
 }
+/* Those with shortwave paths */
+StepPoolFn
+step_most_fn(uint32_t v)
+{
+  switch(v) {
+    case 2u: return k_step_most<2u>;
+    case 3u: return k_step_most<3u>;
+    case 6u: return k_step_most<6u>;
+    default: return k_step_most<7u>;
+  }
+}
+StepPoolFn
+pair_fn(uint32_t v)
+{
+  switch(v) {
+    case 2u: return k_pair<2u>;
+    case 3u: return k_pair<3u>;
+    case 6u: return k_pair<6u>;
+    default: return k_pair<7u>;
+  }
+}
 
 /* Grid of a kernel of `threads' threads a block that fills the device */
 template <class Fn>
 cudaError_t
 step_shape(Fn kern, const PTables& T, uint32_t threads, uint32_t blocks_per_sm, int device, size_t* smem,
-           int* in_smem, unsigned* grid)
+           int* in_smem, unsigned* grid, size_t own = 0)
 {
   const size_t tables = ((T.nscenes * sizeof(DScene) + 15) & ~(size_t)15) + T.nreqs * sizeof(DRequest);
   *in_smem = tables <= 96 * 1024;
-  *smem = step_event_bytes(threads) + (*in_smem ? tables : 0);
+  *smem = (own ? own : step_event_bytes(threads)) + (*in_smem ? tables : 0);
   if(*smem > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem);
     if(e != cudaSuccess) return e;
@@ -247,17 +332,67 @@ step_shape(Fn kern, const PTables& T, uint32_t threads, uint32_t blocks_per_sm, 
 
 }  // namespace
 
+/* The buffer of the last paths of a run (17 MB), one a host thread and device */
+StepBufs&
+thread_last(int device)
+{
+  static thread_local std::map<int, std::unique_ptr<StepBufs>> bufs;
+  std::unique_ptr<StepBufs>& b = bufs[device];
+  if(!b) b = std::make_unique<StepBufs>();
+  return *b;
+}
+
 cudaError_t
-launch_step(const PTables& T, uint32_t block_size, uint32_t blocks_per_sm, int device, cudaStream_t st)
+launch_step(const PTables& T, uint32_t block_size, uint32_t blocks_per_sm, int device, cudaStream_t st,
+            bool may_keep)
 {
   if(!T.total) return cudaSuccess;
-  auto kern = step_fn(T.variant);
   size_t smem;
   int in_smem;
   unsigned grid;
-  const cudaError_t e = step_shape(kern, T, block_size, blocks_per_sm, device, &smem, &in_smem, &grid);
-  if(e != cudaSuccess) return e;
-  kern<<<grid, block_size, smem, st>>>(T, in_smem);
+  cudaError_t e;
+  if(!may_keep || !(T.variant & HV_SW)) {
+    auto kern = step_fn(T.variant);
+    if((e = step_shape(kern, T, block_size, blocks_per_sm, device, &smem, &in_smem, &grid))) return e;
+    kern<<<grid, block_size, smem, st>>>(T, in_smem);
+    note_launches(1);
+    return cudaGetLastError();
+  }
+  /* Shortwave: a lone path's bounce takes 7.5 us in k_pair and 9 in k_step, but
+   * a full device's takes a fifth more, as half of the warps hold no path: a
+   * run that fits in k_pair's lanes goes there (1024 realisations 4.33 -> 3.56
+   * ms), of another only the last paths (all of a flux map of 88 000: 31.4 ms,
+   * its last paths 26.6, none 28.0). */
+  auto pair = pair_fn(T.variant);
+  const uint32_t pair_threads = 64 * kPairs;
+  size_t pair_smem;
+  int pair_in_smem;
+  unsigned pair_grid;
+  if((e = step_shape(pair, T, pair_threads, 0, device, &pair_smem, &pair_in_smem, &pair_grid, pair_bytes())))
+    return e;
+  StepBufs& B = thread_last(device);
+  if(!B.ctl.ptr && !B.ctl.alloc(sizeof(StepCtl))) return cudaErrorMemoryAllocation;
+  if((e = cudaMemsetAsync(B.ctl.ptr, 0, sizeof(StepCtl), st))) return e;
+  StepPool P{};
+  P.ctl = (StepCtl*)B.ctl.ptr;
+  if(T.total > (uint64_t)pair_grid * 32 * kPairs) {
+    auto most = step_most_fn(T.variant);
+    if((e = step_shape(most, T, block_size, blocks_per_sm, device, &smem, &in_smem, &grid))) return e;
+    const uint32_t lanes = grid * block_size;
+    if(B.lanes < lanes) {
+      if(B.paths[0].ptr) { cudaFree(B.paths[0].ptr); B.paths[0].ptr = nullptr; }
+      B.lanes = 0;
+      if(!B.paths[0].alloc((size_t)lanes * kPathV4 * 16)) return cudaErrorMemoryAllocation;
+      B.lanes = lanes;
+    }
+    P.paths[0] = (uint4*)B.paths[0].ptr;
+    P.turn = 1; /* saves into paths[0] */
+    most<<<grid, block_size, smem, st>>>(T, P, in_smem);
+    note_launches(1);
+    if((e = cudaGetLastError())) return e;
+  }
+  P.turn = 0;
+  pair<<<pair_grid, pair_threads, pair_smem, st>>>(T, P, pair_in_smem);
   note_launches(1);
   return cudaGetLastError();
 }

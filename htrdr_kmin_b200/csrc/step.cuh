@@ -61,7 +61,7 @@ step_event_bytes(uint32_t threads)
 /* Runs paths until `work' has no more, or asks to stop: then the lanes' paths
  * are handed to work.save().  Work:
  *   scenes, request(e)  the tables of a path
- *   stop()              whether to stop (warp-uniform)
+ *   stop(n)             whether to stop, with n live paths (warp-uniform)
  *   take(want, p, e)    gives the lanes of `want' a path each, or leaves them
  *                       idle when there is none left (all lanes call it);
  *                       returns whether this lane may ask again
@@ -75,8 +75,8 @@ step_loop(Work& work, PathTrace& p, PathEvent& e, bool drained)
   p.c_seg = p.c_node = p.c_tc = 0;
   p.si = 0;
   for(;;) {
-    if(work.stop()) { work.save(p, e); return; }
     const unsigned live = __ballot_sync(HG_FULL, p.state != ST_IDLE);
+    if(work.stop((uint32_t)__popc(live))) { work.save(p, e); return; }
     const unsigned idle = __ballot_sync(HG_FULL, p.state == ST_IDLE && !drained);
     if(idle && (!live || __popc(idle) >= step_refill(V))) {
       const bool more = work.take(p.state == ST_IDLE && !drained, p, e);

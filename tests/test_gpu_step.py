@@ -1,6 +1,7 @@
-"""The finishing kernel (a lane per path, a warp's paths in step, single-cell
-leaves crossed by a loop of their own) against the plain kernel, where its
-walk can go wrong: grids of a cell or two, leaves larger than a cell, cells
+"""The step loop (a lane per path, a warp's paths in step, single-cell leaves
+crossed by a loop of their own) and the pair kernel (a path's sun
+transmissivity on a second warp) against the plain kernel, where the walk and
+the pair's guess of the random stream can go wrong: grids of a cell or two, leaves larger than a cell, cells
 that straddle gas layers (null collisions), negative coordinates and tiles,
 horizontal rays, every axis consecutive in the majorant grid, and majorants
 whose sign cannot mark a leaf.
@@ -58,20 +59,39 @@ CASES = {
 }
 
 
+# 777 realisations: the pair kernel alone; 25 300: the step loop, the last paths
+# handed to the pair kernel
+@pytest.mark.parametrize("size", [(37, 21), (220, 115)])
 @pytest.mark.parametrize("name", list(CASES))
-def test_step_kernel_equals_plain(gpu_lib, name):
+def test_step_kernels_equal_plain(gpu_lib, name, size):
     skw, rkw = CASES[name]
     lw = skw.get("lw", False)
     gs = gpu_lib.GpuScene(_scene(**skw))
-    req = _request(lw, **rkw)
+    req = _request(lw, **{**rkw, "width": size[0], "height": size[1]})
     w = gs.realisation_weights(req, 0, req.width * req.height).ravel()
-    t = gpu_lib.mode_tuning(req.mode)
-    t.wave_tail = 1 << 30  # the whole run in the finishing kernel
-    gs.set_engine(gpu_lib.ENGINE_WAVEFRONT, t)
     buf, st = gs.draw_map(req)
     got = (buf["sum"] if req.mode == S.MODE_FLUX_SW else buf["L"]).ravel()
     assert st["failures"] == 0 and np.count_nonzero(w) > w.size // 8
     np.testing.assert_allclose(got, w, rtol=1e-12, atol=0)
+
+
+@pytest.mark.parametrize("name", ["straddles_layers", "large_leaves", "not_repeated"])
+def test_radiance_kernels_agree(gpu_lib, name):
+    """A ray's radiance does not depend on how many rays the call has: the pair
+    kernel (few rays) and the step loop (many)."""
+    gs = gpu_lib.GpuScene(_scene(**CASES[name][0]))
+    rng = np.random.default_rng(2)
+    n = 45000
+    pos = rng.uniform((0, 0, 1), (1800, 1300, 2500), (n, 3))
+    d = rng.standard_normal((n, 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    band = rng.integers(0, 2, n).astype(np.uint32)
+    quad = rng.integers(0, 2, n).astype(np.uint32)
+    wlen = 525.0 + 50.0 * band
+    many = gs.radiance_sw(pos, d, wlen, band, quad, seed=4)
+    for k in (1, 33, 6000):
+        few = gs.radiance_sw(pos[:k], d[:k], wlen[:k], band[:k], quad[:k], seed=4)
+        np.testing.assert_allclose(few, many[:k], rtol=1e-12, atol=0)
 
 
 def test_negative_majorants_take_the_general_voxel(gpu_lib):

@@ -514,7 +514,7 @@ def mode_tuning(mode: int) -> Tuning:
 
 
 def draw_maps_batched(items: Sequence[tuple], tuning: Optional[Tuning] = None):
-    """Run many (GpuScene, Request) in one persistent kernel.  Returns the list
+    """Run many (GpuScene, Request) from one work queue.  Returns the list
     of pixel buffers and the stats of the launch."""
     n = len(items)
     arr = (BatchItem * n)()

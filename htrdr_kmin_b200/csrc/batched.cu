@@ -427,7 +427,7 @@ try {
 HG_API_CATCH("htrdr_gpu_autotune")
 
 /*******************************************************************************
- * Reusable batch: the whole launch sequence (clear, persistent kernel,
+ * Reusable batch: the whole launch sequence (clear, step loop,
  * finalize of every item) captured once in a CUDA graph and replayed.
  ******************************************************************************/
 struct htrdr_gpu_batch {
@@ -461,7 +461,7 @@ htrdr_gpu_batch_create(const htrdr_gpu_batch_item* items, size_t n, const htrdr_
 try {
   if(!items || !n || !out) return HTRDR_GPU_RES_BAD_ARG;
   htrdr_gpu_tuning tun = items_tuning(items, n, tuning);
-  if(!tuning) tun.engine = HTRDR_GPU_ENGINE_PERSISTENT; /* a mode default may name the wavefront */
+  if(!tuning) tun.engine = HTRDR_GPU_ENGINE_PERSISTENT; /* a mode default names the wavefront */
   if(!valid_tuning(tun)) return HTRDR_GPU_RES_BAD_ARG;
   if(tun.engine != HTRDR_GPU_ENGINE_PERSISTENT && tun.engine != HTRDR_GPU_ENGINE_SORTED) {
     set_error("graph batches run the persistent engines");
@@ -503,7 +503,7 @@ try {
   float k = 0, t = 0;
   cudaEventElapsedTime(&k, b->e1, b->e2);
   cudaEventElapsedTime(&t, b->e0, b->e3);
-  read_stats(c, k, t, 1 + b->items.size(), stats); /* persistent kernel + finalizes */
+  read_stats(c, k, t, 1 + b->items.size(), stats); /* k_step + finalizes */
   return HTRDR_GPU_RES_OK;
 }
 HG_API_CATCH("htrdr_gpu_batch_run")

@@ -199,9 +199,7 @@ sorted_lists_bytes(uint32_t threads)
  * slots that any lane may run, so every step the block sorts its slots by
  * stage -- tracing, or waiting for an event (or for new work) -- into two
  * lists, and lanes 0..n-1 take the n entries of each list in turn.  The
- * warps of each pass are therefore full of lanes in the same stage (the
- * ballot regrouping of persistent_loop only gathers the lanes a warp owns),
- * and warps past the end of a list skip it.  `regroup_period' voxel steps are
+ * warps of each pass are therefore full of lanes in the same stage, and warps past the end of a list skip it.  `regroup_period' voxel steps are
  * taken per trace visit.  Same state machine, same streams, same weights. */
 template <unsigned V>
 __device__ __forceinline__ void

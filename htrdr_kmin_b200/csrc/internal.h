@@ -171,7 +171,7 @@ cudaError_t launch_sample_wavelength(const DRequest& R, int channel, size_t n, c
                                      const double* r1, uint32_t* cb, double* wlen, double* pdf,
                                      cudaStream_t st);
 
-/* Persistent engine (batched.cu).  A launch covers items, each a range of
+/* Work queue (batched.cu).  A launch covers items, each a range of
  * realisations [begin, begin + count) of one request; the realisations of
  * all items form one work queue. */
 struct PItem {
@@ -204,7 +204,7 @@ tables_variant(const std::vector<DScene>& scenes, const std::vector<DRequest>& r
 cudaError_t launch_sorted(const PTables& T, uint32_t block_size, uint32_t blocks_per_sm, int device,
                           cudaStream_t st);
 bool valid_tuning(const htrdr_gpu_tuning& t);
-/* One request on the persistent engine.  `tables' (device memory of
+/* One request on a work-queue engine.  `tables' (device memory of
  * single_tables_bytes()) receives the launch's scene/request/item tables;
  * `cnt' (device, 128 bytes) holds the counters and the queue head and must be
  * zeroed before the launch. */

@@ -5,7 +5,7 @@
  *   1. admits pending requests in arrival order while their device memory
  *      (FP64 accumulators + output staging) fits in the HBM budget; the
  *      accumulators stay resident until the request completes;
- *   2. launches rounds of the persistent kernel, each over a share of the
+ *   2. launches rounds of the step loop, each over a share of the
  *      not-yet-dispatched realisations of every admitted request; up to
  *      `kDepth' rounds are in flight on their own streams, so the next round
  *      fills the SMs that the slow paths of the previous one leave idle, and

@@ -5,7 +5,7 @@
  * path_event() (sensor sampling, scattering/surface events, sun next-event
  * estimation, accumulation) and trace_step() (one voxel of a delta-tracking
  * trace).  The same code runs in the one-thread-per-realisation kernel and in
- * the persistent batched kernel, so both produce the same weight for a given
+ * the step loop, so both produce the same weight for a given
  * (pixel, realisation).
  *
  * Reference behaviour restated here:

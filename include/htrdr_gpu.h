@@ -191,8 +191,8 @@ enum htrdr_gpu_engine {
   HTRDR_GPU_ENGINE_PERSISTENT = 0,
   HTRDR_GPU_ENGINE_PLAIN = 1,
   HTRDR_GPU_ENGINE_WAVEFRONT = 2,
-  /* the persistent kernel with its paths in shared memory, regrouped by
-   * stage across the whole block at every step */
+  /* a kernel with its paths in shared memory, regrouped by stage
+   * across the whole block at every step */
   HTRDR_GPU_ENGINE_SORTED = 3
 };
 struct htrdr_gpu_tuning;
@@ -311,7 +311,7 @@ htrdr_gpu_sample_wavelength(struct htrdr_gpu_scene* scene, const struct htrdr_gp
                             int channel, size_t n, const double* r0, const double* r1,
                             uint32_t* cdf_band, double* wlen, double* pdf);
 
-/* ---- batched engine: many requests in one persistent kernel ---- */
+/* ---- batched engine: many requests in one work queue ---- */
 struct htrdr_gpu_batch_item {
   struct htrdr_gpu_scene* scene;
   struct htrdr_gpu_request req;
@@ -329,8 +329,8 @@ struct htrdr_gpu_tuning {
   uint32_t trace_budget;  /* not used */
   uint32_t wave_tail;     /* not used */
 };
-/* Renders every item (each one htrdr_draw_map call of the reference) in one
- * persistent kernel; item buffers are host memory.  tuning == NULL: the
+/* Renders every item (each one htrdr_draw_map call of the reference) from one
+ * work queue; item buffers are host memory.  tuning == NULL: the
  * default of the items' modes (htrdr_gpu_mode_tuning; SW/CIE wins when mixed). */
 HTRDR_GPU_API htrdr_gpu_res_T
 htrdr_gpu_draw_maps_batched(struct htrdr_gpu_batch_item* items, size_t n,
@@ -374,7 +374,7 @@ HTRDR_GPU_API void htrdr_gpu_batch_release(struct htrdr_gpu_batch* batch);
  * A scheduling thread admits them while their device memory (FP64
  * accumulators + output staging) fits in the HBM budget, keeps their
  * accumulators resident, and feeds a fair share of every admitted request's
- * remaining realisations to the engine: rounds of the persistent kernel, or
+ * remaining realisations to the engine: rounds of the step loop, or
  * a pool of paths in flight, whose lanes take the realisations of newly
  * admitted requests as soon as their paths end.  Requests that arrive while
  * others render join the running work.  A request completes when all its

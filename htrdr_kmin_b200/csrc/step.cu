@@ -309,22 +309,27 @@ pair_fn(uint32_t v)
   }
 }
 
-/* Grid of a kernel of `threads' threads a block that fills the device */
+/* Grid of a kernel of `*threads' threads a block that fills the device; blocks
+ * that its registers do not allow become the largest that they do */
 template <class Fn>
 cudaError_t
-step_shape(Fn kern, const PTables& T, uint32_t threads, uint32_t blocks_per_sm, int device, size_t* smem,
+step_shape(Fn kern, const PTables& T, uint32_t* threads, uint32_t blocks_per_sm, int device, size_t* smem,
            int* in_smem, unsigned* grid, size_t own = 0)
 {
+  cudaFuncAttributes attr;
+  const cudaError_t ea = cudaFuncGetAttributes(&attr, kern);
+  if(ea != cudaSuccess) return ea;
+  *threads = std::min(*threads, (uint32_t)attr.maxThreadsPerBlock & ~31u);
   const size_t tables = ((T.nscenes * sizeof(DScene) + 15) & ~(size_t)15) + T.nreqs * sizeof(DRequest);
   *in_smem = tables <= 96 * 1024;
-  *smem = (own ? own : step_event_bytes(threads)) + (*in_smem ? tables : 0);
+  *smem = (own ? own : step_event_bytes(*threads)) + (*in_smem ? tables : 0);
   if(*smem > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem);
     if(e != cudaSuccess) return e;
   }
   int nsm = 0, per_sm = 0;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (int)threads, *smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (int)*threads, *smem);
   if(blocks_per_sm) per_sm = std::min(per_sm, (int)blocks_per_sm);
   *grid = (unsigned)(nsm * std::max(per_sm, 1));
   return cudaSuccess;
@@ -353,7 +358,7 @@ launch_step(const PTables& T, uint32_t block_size, uint32_t blocks_per_sm, int d
   cudaError_t e;
   if(!may_keep || !(T.variant & HV_SW)) {
     auto kern = step_fn(T.variant);
-    if((e = step_shape(kern, T, block_size, blocks_per_sm, device, &smem, &in_smem, &grid))) return e;
+    if((e = step_shape(kern, T, &block_size, blocks_per_sm, device, &smem, &in_smem, &grid))) return e;
     kern<<<grid, block_size, smem, st>>>(T, in_smem);
     note_launches(1);
     return cudaGetLastError();
@@ -364,11 +369,11 @@ launch_step(const PTables& T, uint32_t block_size, uint32_t blocks_per_sm, int d
    * ms), of another only the last paths (all of a flux map of 88 000: 31.4 ms,
    * its last paths 26.6, none 28.0). */
   auto pair = pair_fn(T.variant);
-  const uint32_t pair_threads = 64 * kPairs;
+  uint32_t pair_threads = 64 * kPairs;
   size_t pair_smem;
   int pair_in_smem;
   unsigned pair_grid;
-  if((e = step_shape(pair, T, pair_threads, 0, device, &pair_smem, &pair_in_smem, &pair_grid, pair_bytes())))
+  if((e = step_shape(pair, T, &pair_threads, 0, device, &pair_smem, &pair_in_smem, &pair_grid, pair_bytes())))
     return e;
   StepBufs& B = thread_last(device);
   if(!B.ctl.ptr && !B.ctl.alloc(sizeof(StepCtl))) return cudaErrorMemoryAllocation;
@@ -377,7 +382,7 @@ launch_step(const PTables& T, uint32_t block_size, uint32_t blocks_per_sm, int d
   P.ctl = (StepCtl*)B.ctl.ptr;
   if(T.total > (uint64_t)pair_grid * 32 * kPairs) {
     auto most = step_most_fn(T.variant);
-    if((e = step_shape(most, T, block_size, blocks_per_sm, device, &smem, &in_smem, &grid))) return e;
+    if((e = step_shape(most, T, &block_size, blocks_per_sm, device, &smem, &in_smem, &grid))) return e;
     const uint32_t lanes = grid * block_size;
     if(B.lanes < lanes) {
       if(B.paths[0].ptr) { cudaFree(B.paths[0].ptr); B.paths[0].ptr = nullptr; }
@@ -404,7 +409,7 @@ step_capacity(uint32_t block_size, uint32_t blocks_per_sm, int device)
   size_t smem;
   int in_smem;
   unsigned grid;
-  if(step_shape(k_step<HV_ALL>, T, block_size, blocks_per_sm, device, &smem, &in_smem, &grid)) return 0;
+  if(step_shape(k_step<HV_ALL>, T, &block_size, blocks_per_sm, device, &smem, &in_smem, &grid)) return 0;
   return (uint64_t)grid * block_size;
 }
 
@@ -439,12 +444,13 @@ step_pool_launch(const PTables& T, StepBufs& B, uint64_t ns, uint32_t blocks_per
   P.lanes = B.lanes;
   P.ns = ns;
   auto kern = step_pool_fn(T.variant);
+  uint32_t threads = kPoolThreads;
   size_t smem;
   int in_smem;
   unsigned grid;
-  const cudaError_t e = step_shape(kern, T, kPoolThreads, blocks_per_sm, device, &smem, &in_smem, &grid);
+  const cudaError_t e = step_shape(kern, T, &threads, blocks_per_sm, device, &smem, &in_smem, &grid);
   if(e != cudaSuccess) return e;
-  kern<<<grid, kPoolThreads, smem, st>>>(T, P, in_smem);
+  kern<<<grid, threads, smem, st>>>(T, P, in_smem);
   k_step_turn<<<1, 1, 0, st>>>(T, P.ctl, B.turn);
   B.turn ^= 1u;
   note_launches(2);

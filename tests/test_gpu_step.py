@@ -75,6 +75,20 @@ def test_step_kernels_equal_plain(gpu_lib, name, size):
     np.testing.assert_allclose(got, w, rtol=1e-12, atol=0)
 
 
+# more threads than a shortwave block has registers for, and a single warp
+@pytest.mark.parametrize("block", [32, 288, 512])
+@pytest.mark.parametrize("name", ["straddles_layers", "lw"])
+def test_block_sizes(gpu_lib, name, block):
+    skw, rkw = CASES[name]
+    gs = gpu_lib.GpuScene(_scene(**skw))
+    req = _request(skw.get("lw", False), **{**rkw, "width": 220, "height": 115})
+    want = gs.draw_map(req)[0]["L"].ravel()
+    tuning = gpu_lib.mode_tuning(req.mode)
+    tuning.block_size = block
+    got = gpu_lib.draw_maps_batched([(gs, req)], tuning)[0][0]["L"].ravel()
+    np.testing.assert_array_equal(got, want)
+
+
 @pytest.mark.parametrize("name", ["straddles_layers", "large_leaves", "not_repeated"])
 def test_radiance_kernels_agree(gpu_lib, name):
     """A ray's radiance does not depend on how many rays the call has: the pair

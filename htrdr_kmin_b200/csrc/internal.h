@@ -219,10 +219,11 @@ cudaError_t launch_step(const PTables& T, uint32_t block_size, uint32_t blocks_p
 uint64_t step_capacity(uint32_t block_size, uint32_t blocks_per_sm, int device);
 
 /* Serving pool: launches that end after `ns' with their live paths saved.
- * `paths' are read and written in turn; n[i] paths are saved in paths[i]. */
+ * `paths' are read and written in turn; n[i] paths are saved in paths[i],
+ * never more than its room of `lanes'. */
 struct StepCtl {
   uint32_t n[2];
-  uint32_t fetch; /* next saved path to take */
+  uint32_t fetch; /* saved paths taken */
   uint32_t pad;
 };
 struct StepPool {
@@ -233,7 +234,7 @@ struct StepPool {
 };
 struct StepBufs {
   DevBuf paths[2], ctl;
-  uint32_t lanes = 0; /* paths in flight at most */
+  uint32_t lanes = 0; /* paths in flight at most: room of each of `paths' */
   uint32_t turn = 0;  /* paths[turn] holds the saved ones */
 };
 bool step_pool_create(StepBufs& B, uint32_t lanes, int device, cudaStream_t st);

@@ -532,6 +532,7 @@ htrdr_gpu_server::loop_wave()
     const Readback* rb = (const Readback*)w_rb[b];
     dev_next = rb_epoch[b] == epoch ? rb->next : 0; /* else: nothing known taken yet */
     dev_live = rb->ctl.n[rb_turn[b]];
+    if(dev_live > pool.lanes) { set_error("server: more paths saved than the pool holds"); return false; }
     for(SReq* r : active) {
       /* a read-back issued before the request was admitted holds another
        * request's count in its table slot */

@@ -66,7 +66,7 @@ struct QueueWork {
   const uint4* in;
   uint4* out;
   StepCtl* ctl;
-  uint32_t n_in, turn;
+  uint32_t n_in, turn, room;
   unsigned long long until;
   bool saved_left, dry;
 
@@ -91,7 +91,8 @@ struct QueueWork {
         if(m & (1u << lane)) {
           const uint32_t i = i0 + __popc(m & ((1u << lane) - 1u));
           if(i < n_in) {
-            load_path(p, e, in + (size_t)i * kPathV4);
+            /* from the end: first those that the launch before left */
+            load_path(p, e, in + (size_t)(n_in - 1 - i) * kPathV4);
             p.t0 = gtimer() - p.t0; /* saved: busy time so far */
             want = false;
           } else {
@@ -123,31 +124,24 @@ struct QueueWork {
     sums->add(p);
   }
 
-  /* The warp's paths to the pool, and the saved ones that no lane took */
+  /* The warp's paths to the pool.  They fit: a lane holds one path, and takes
+   * one from the queue only when no saved path is left, so a launch that took
+   * from the queue has every path it saves in one of its `lanes' lanes, and one
+   * that did not has as many as it read.  (Saved paths that no lane took stay
+   * where they are until the launch has ended, in whatever order its blocks
+   * start and end: k_step_turn.) */
   __device__ __forceinline__ void save(PathTrace& p, PathEvent& e)
   {
     if(Kind != WK_POOL && Kind != WK_LAST_OUT) return;
     const unsigned lane = threadIdx.x & 31u;
-    bool keep = p.state != ST_IDLE;
-    for(;;) {
-      const unsigned m = __ballot_sync(HG_FULL, keep);
-      uint32_t o = 0;
-      if(lane == 0 && m) o = atomicAdd(&ctl->n[turn ^ 1u], (uint32_t)__popc(m));
-      o = __shfl_sync(HG_FULL, o, 0);
-      if(keep) {
-        p.t0 = gtimer() - p.t0;
-        save_path(p, e, out + (size_t)(o + __popc(m & ((1u << lane) - 1u))) * kPathV4);
-      }
-      if(!kReads) return;
-      uint32_t i0 = 0;
-      if(lane == 0) i0 = atomicAdd(&ctl->fetch, 32u);
-      i0 = __shfl_sync(HG_FULL, i0, 0);
-      if(i0 >= n_in) return;
-      keep = i0 + lane < n_in;
-      if(keep) {
-        load_path(p, e, in + (size_t)(i0 + lane) * kPathV4);
-        p.t0 = gtimer() - p.t0;
-      }
+    const bool keep = p.state != ST_IDLE;
+    const unsigned m = __ballot_sync(HG_FULL, keep);
+    uint32_t o = 0;
+    if(lane == 0 && m) o = atomicAdd(&ctl->n[turn ^ 1u], (uint32_t)__popc(m));
+    o = __shfl_sync(HG_FULL, o, 0) + __popc(m & ((1u << lane) - 1u));
+    if(keep && o < room) { /* else: counted, for the host to see */
+      p.t0 = gtimer() - p.t0;
+      save_path(p, e, out + (size_t)o * kPathV4);
     }
   }
 };
@@ -178,7 +172,8 @@ queue_work(const PTables& T, StepSums* sums, const StepPool& P)
     work.out = P.paths[P.turn ^ 1u];
     work.ctl = P.ctl;
     work.turn = P.turn;
-    work.n_in = work.kReads ? P.ctl->n[P.turn] : 0u;
+    work.room = P.lanes;
+    work.n_in = work.kReads ? min(P.ctl->n[P.turn], P.lanes) : 0u;
     work.until = gtimer() + P.ns;
     work.saved_left = work.n_in != 0;
   }
@@ -263,13 +258,30 @@ k_pair(PTables T, StepPool P, int tables_in_smem)
   if(threadIdx.x == 0) flush_sums(T, sums);
 }
 
-/* After a launch of a pool: the paths it read are free, and the queue's head
- * goes back to the queued total, so that work appended later starts there */
+/* After a launch of a pool: the saved paths that no lane took join those it
+ * saved, those it read are free, and the queue's head goes back to the queued
+ * total, so that work appended later starts there.  Paths are left over where
+ * blocks of the launch started late (another stream held their SMs) or where
+ * it had fewer lanes than the one before it (another variant): the launch's own
+ * blocks cannot move them, as a lane that has yet to start would take work from
+ * the queue beside them.  One block: there is nothing to move most often, and
+ * 38 000 paths at most. */
 __global__ void
-k_step_turn(PTables T, StepCtl* ctl, uint32_t read)
+k_step_turn(PTables T, StepPool P)
 {
-  ctl->n[read] = 0;
-  ctl->fetch = 0;
+  const uint32_t n_in = min(P.ctl->n[P.turn], P.lanes);
+  const uint32_t taken = min(P.ctl->fetch, n_in), at = P.ctl->n[P.turn ^ 1u];
+  const uint32_t left = n_in - taken;
+  if(at + left <= P.lanes) {
+    const uint4* from = P.paths[P.turn];
+    uint4* to = P.paths[P.turn ^ 1u] + (size_t)at * kPathV4;
+    for(uint32_t i = threadIdx.x; i < left * kPathV4; i += blockDim.x) to[i] = from[i];
+  }
+  __syncthreads();
+  if(threadIdx.x) return;
+  P.ctl->n[P.turn] = 0;
+  P.ctl->n[P.turn ^ 1u] = at + left;
+  P.ctl->fetch = 0;
   queue_clamp(T);
 }
 
@@ -392,6 +404,7 @@ launch_step(const PTables& T, uint32_t block_size, uint32_t blocks_per_sm, int d
     }
     P.paths[0] = (uint4*)B.paths[0].ptr;
     P.turn = 1; /* saves into paths[0] */
+    P.lanes = B.lanes;
     most<<<grid, block_size, smem, st>>>(T, P, in_smem);
     note_launches(1);
     if((e = cudaGetLastError())) return e;
@@ -451,7 +464,7 @@ step_pool_launch(const PTables& T, StepBufs& B, uint64_t ns, uint32_t blocks_per
   const cudaError_t e = step_shape(kern, T, &threads, blocks_per_sm, device, &smem, &in_smem, &grid);
   if(e != cudaSuccess) return e;
   kern<<<grid, threads, smem, st>>>(T, P, in_smem);
-  k_step_turn<<<1, 1, 0, st>>>(T, P.ctl, B.turn);
+  k_step_turn<<<1, 1024, 0, st>>>(T, P);
   B.turn ^= 1u;
   note_launches(2);
   return cudaGetLastError();

@@ -218,13 +218,15 @@ cudaError_t launch_step(const PTables& T, uint32_t block_size, uint32_t blocks_p
 /* Threads that launch keeps resident on the device */
 uint64_t step_capacity(uint32_t block_size, uint32_t blocks_per_sm, int device);
 
-/* Serving pool: launches that end after `ns' with their live paths saved.
+/* Serving pool: launches that end `ns' after their first block started, with
+ * their live paths saved.
  * `paths' are read and written in turn; n[i] paths are saved in paths[i],
  * never more than its room of `lanes'. */
 struct StepCtl {
   uint32_t n[2];
   uint32_t fetch; /* saved paths taken */
   uint32_t pad;
+  unsigned long long until; /* end of the launch that runs (0: none has started) */
 };
 struct StepPool {
   uint4* paths[2];

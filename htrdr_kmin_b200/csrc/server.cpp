@@ -360,8 +360,9 @@ htrdr_gpu_server::loop()
  * launch, tell when a request's map is complete (finalize, copy to the host
  * buffer).
  ******************************************************************************/
-/* Saving and resuming a full pool takes ~20 us: 1 % of a launch */
-static constexpr uint64_t kLaunchNs = 2000000;
+/* Length of a launch in ns: saving and resuming a full pool takes ~20 us, 1 %
+ * of the longest; the shortest holds a bounce of every path */
+static constexpr double kLaunchNs = 2e6, kLaunchNsMin = 1e5;
 
 bool
 htrdr_gpu_server::wave_setup()
@@ -580,10 +581,10 @@ htrdr_gpu_server::loop_wave()
   auto launch = [&](int b) -> bool {
     Readback* rb = (Readback*)w_rb[b];
     const PTables T = wave_tables_now();
+    const uint64_t ns = (uint64_t)std::max(kLaunchNsMin, std::min(kLaunchNs, cfg.round_target_ms * 1e6));
     const bool ok =
       cuda_ok(cudaEventRecord(w_ta[b], io), "event")
-      && cuda_ok(step_pool_launch(T, pool, std::min<uint64_t>(kLaunchNs, (uint64_t)(cfg.round_target_ms * 1e6)),
-                                  cfg.tuning.blocks_per_sm, cfg.device, io), "k_step_pool")
+      && cuda_ok(step_pool_launch(T, pool, ns, cfg.tuning.blocks_per_sm, cfg.device, io), "k_step_pool")
       && cuda_ok(cudaEventRecord(w_tb[b], io), "event")
       && cuda_ok(cudaMemcpyAsync(&rb->ctl, pool.ctl.ptr, sizeof(StepCtl), cudaMemcpyDeviceToHost, io), "D2H")
       && cuda_ok(cudaMemcpyAsync(&rb->next, (char*)w_cnt.ptr + 64, 8, cudaMemcpyDeviceToHost, io), "D2H")

@@ -45,7 +45,7 @@ save_path(const PathTrace& p, const PathEvent& e, uint4* v)
 
 /* Where a launch's paths come from and go to: the queue alone; a pool, whose
  * saved paths come before the queue and which saves the live ones when the
- * launch's time is over; the queue, and the last paths saved for another
+ * launch's time is over (launch_end); the queue, and the last paths saved for another
  * launch when it has run dry (LAST_OUT) and taken up by that one (LAST_IN) */
 enum { WK_QUEUE = 0, WK_POOL, WK_LAST_OUT, WK_LAST_IN };
 
@@ -62,19 +62,24 @@ struct QueueWork {
   const DScene* scenes;
   PTables T;
   StepSums* sums;
-  /* Pool: saved paths read and written, their counters, the end of the launch */
+  /* Pool: saved paths read and written, their counters, the end of the launch,
+   * whether this block started before it and has not taken its first turn */
   const uint4* in;
   uint4* out;
   StepCtl* ctl;
   uint32_t n_in, turn, room;
   unsigned long long until;
-  bool saved_left, dry;
+  bool saved_left, dry, fresh;
 
   __device__ __forceinline__ const DRequest& request(const PathEvent& e) const { return T.reqs[e.ri]; }
 
   __device__ __forceinline__ bool stop(uint32_t live)
   {
-    if(Kind == WK_POOL) return __shfl_sync(HG_FULL, (int)(gtimer() >= until), 0) != 0;
+    if(Kind == WK_POOL) {
+      const bool over = __shfl_sync(HG_FULL, (int)(gtimer() >= until), 0) != 0 && !fresh;
+      fresh = false;
+      return over;
+    }
     return Kind == WK_LAST_OUT && live <= kLastPaths && __any_sync(HG_FULL, dry);
   }
 
@@ -159,7 +164,7 @@ lane_unused(const PTables& T, uint32_t saved, uint32_t warps_per_block)
 
 template <int Kind>
 __device__ __forceinline__ QueueWork<Kind>
-queue_work(const PTables& T, StepSums* sums, const StepPool& P)
+queue_work(const PTables& T, StepSums* sums, const StepPool& P, unsigned long long until = 0, bool fresh = true)
 {
   QueueWork<Kind> work;
   work.T = T;
@@ -174,7 +179,8 @@ queue_work(const PTables& T, StepSums* sums, const StepPool& P)
     work.turn = P.turn;
     work.room = P.lanes;
     work.n_in = work.kReads ? min(P.ctl->n[P.turn], P.lanes) : 0u;
-    work.until = gtimer() + P.ns;
+    work.until = until;
+    work.fresh = fresh;
     work.saved_left = work.n_in != 0;
   }
   return work;
@@ -191,6 +197,18 @@ flush_sums(const PTables& T, const StepSums& sums)
   atomicAdd(&c->fail, sums.fail);
 }
 
+/* The end of a pool's launch, the same for all of its blocks: counted from the
+ * first one that starts.  A block that starts after it takes nothing; the first
+ * one always takes a turn, so a launch advances whatever its length. */
+__device__ __forceinline__ unsigned long long
+launch_end(const StepPool& P, bool* in_time)
+{
+  const unsigned long long now = gtimer(), mine = now + P.ns;
+  const unsigned long long first = atomicCAS(&P.ctl->until, 0ull, mine);
+  *in_time = !first || now < first;
+  return first ? first : mine;
+}
+
 template <unsigned V, int Kind>
 __device__ __forceinline__ void
 step_block(PTables& T, const StepPool& P, int tables_in_smem)
@@ -198,10 +216,16 @@ step_block(PTables& T, const StepPool& P, int tables_in_smem)
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ StepSums sums;
   const bool unused = lane_unused(T, QueueWork<Kind>::kReads ? P.ctl->n[P.turn] : 0u, blockDim.x >> 5);
-  if(threadIdx.x == 0) sums = StepSums{0, 0, 0, 0, 0};
+  __shared__ unsigned long long until;
+  __shared__ bool fresh;
+  if(threadIdx.x == 0) {
+    sums = StepSums{0, 0, 0, 0, 0};
+    if(Kind == WK_POOL) until = launch_end(P, &fresh);
+  }
   if(tables_in_smem) tables_to_smem(T, smem + step_event_bytes(blockDim.x));
   __syncthreads();
-  QueueWork<Kind> work = queue_work<Kind>(T, &sums, P);
+  QueueWork<Kind> work = Kind == WK_POOL ? queue_work<Kind>(T, &sums, P, until, fresh)
+                                         : queue_work<Kind>(T, &sums, P);
   PathTrace p;
   const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
   step_loop<V>(work, p, ((PathEvent*)smem)[threadIdx.x], unused || (Kind == WK_POOL && id >= P.lanes));
@@ -282,6 +306,7 @@ k_step_turn(PTables T, StepPool P)
   P.ctl->n[P.turn] = 0;
   P.ctl->n[P.turn ^ 1u] = at + left;
   P.ctl->fetch = 0;
+  P.ctl->until = 0;
   queue_clamp(T);
 }
 

@@ -77,3 +77,15 @@ def test_pool_beside_other_calls(gpu_lib, slots):
     assert st["failed"] == 0 and maps
     for m in maps:
         _same(m, want, rq.mode)
+
+
+@pytest.mark.parametrize("target_ms", [1e-5, 1e9])
+def test_pool_advances_whatever_the_round_target(gpu_lib, target_ms):
+    api = gpu_lib
+    reqs = _requests(api)[:6]
+    srv = _pool(api, round_target_ms=target_ms)
+    tickets = [srv.submit(*it) for it in reqs]
+    out = [srv.wait(t, WAIT_S) for t in tickets]
+    srv.close()
+    for (gs, r), a in zip(reqs, out):
+        _same(a, gs.draw_map(r)[0], r.mode)

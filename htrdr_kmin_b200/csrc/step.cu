@@ -4,6 +4,7 @@
  * serving pool, whose launches end after a set time with the live paths
  * saved, so that newly admitted requests join them in the next one. */
 #include "pair.cuh"
+#include "spread.h"
 
 #include <algorithm>
 #include <map>
@@ -151,15 +152,15 @@ struct QueueWork {
   }
 };
 
-/* Whether this lane stays empty: few paths are spread over all warps, as a
- * warp with a single path takes its bounces fastest */
+/* Whether this lane stays empty (warp_lanes); the warps are counted across the
+ * blocks first, so that a pool of few paths runs on all SMs */
 __device__ __forceinline__ bool
-lane_unused(const PTables& T, uint32_t saved, uint32_t warps_per_block)
+lane_unused(const PTables& T, uint32_t saved, uint32_t warp, uint32_t warps_per_block, uint64_t room)
 {
   const unsigned long long next = *(volatile unsigned long long*)T.next;
   const unsigned long long left = saved + (T.total > next ? T.total - next : 0ull);
-  const unsigned long long warps = (unsigned long long)gridDim.x * warps_per_block;
-  return (threadIdx.x & 31u) >= (left + warps - 1) / warps;
+  return (threadIdx.x & 31u) >= warp_lanes((uint64_t)warp * gridDim.x + blockIdx.x,
+                                           (uint64_t)gridDim.x * warps_per_block, room, left);
 }
 
 template <int Kind>
@@ -215,7 +216,8 @@ step_block(PTables& T, const StepPool& P, int tables_in_smem)
 {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ StepSums sums;
-  const bool unused = lane_unused(T, QueueWork<Kind>::kReads ? P.ctl->n[P.turn] : 0u, blockDim.x >> 5);
+  const bool unused = lane_unused(T, QueueWork<Kind>::kReads ? P.ctl->n[P.turn] : 0u, threadIdx.x >> 5,
+                                  blockDim.x >> 5, Kind == WK_POOL ? P.lanes : UINT64_MAX);
   __shared__ unsigned long long until;
   __shared__ bool fresh;
   if(threadIdx.x == 0) {
@@ -227,8 +229,7 @@ step_block(PTables& T, const StepPool& P, int tables_in_smem)
   QueueWork<Kind> work = Kind == WK_POOL ? queue_work<Kind>(T, &sums, P, until, fresh)
                                          : queue_work<Kind>(T, &sums, P);
   PathTrace p;
-  const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
-  step_loop<V>(work, p, ((PathEvent*)smem)[threadIdx.x], unused || (Kind == WK_POOL && id >= P.lanes));
+  step_loop<V>(work, p, ((PathEvent*)smem)[threadIdx.x], unused);
   __syncthreads();
   if(threadIdx.x == 0) flush_sums(T, sums);
 }
@@ -265,7 +266,7 @@ k_pair(PTables T, StepPool P, int tables_in_smem)
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ StepSums sums;
   __shared__ uint32_t live[kPairs];
-  const bool unused = lane_unused(T, P.ctl->n[P.turn], kPairs);
+  const bool unused = lane_unused(T, P.ctl->n[P.turn], (threadIdx.x >> 5) % kPairs, kPairs, UINT64_MAX);
   if(threadIdx.x == 0) sums = StepSums{0, 0, 0, 0, 0};
   PairJob* jobs = (PairJob*)(smem + step_event_bytes(32 * kPairs));
   if(tables_in_smem) tables_to_smem(T, smem + pair_bytes());

@@ -61,8 +61,7 @@ launch_sorted(const PTables& T, uint32_t block_size, uint32_t blocks_per_sm, int
   auto kern = sorted_fn(T.variant);
   if(smem > 227 * 1024) return cudaErrorInvalidConfiguration; /* block too large for its paths */
   if(smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem);
+    const cudaError_t e = allow_shared((const void*)kern, device);
     if(e != cudaSuccess) return e;
   }
   int nsm = 0, per_sm = 0;

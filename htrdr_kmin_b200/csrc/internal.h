@@ -210,6 +210,11 @@ bool valid_tuning(const htrdr_gpu_tuning& t);
  * zeroed before the launch. */
 size_t single_tables_bytes();
 
+/* Lets the launches of a kernel use all the shared memory of a block, once for
+ * each device.  The limit belongs to the kernel, whichever thread launches it:
+ * were it set to each launch's own size, two threads could lower it under one
+ * another's launches. */
+cudaError_t allow_shared(const void* kern, int device);
 /* Step loop (step.cu): all queued realisations of T.  may_keep: the calling
  * thread's buffer for the last paths may be used (not by launches that overlap
  * others of the thread, nor by captured ones) */

@@ -389,7 +389,7 @@ launch_radiance(const DScene& S, const RayArgs& a, int device, cudaStream_t st)
    * rays under a cloud 16.5 ms, 24.4 in the step loop */
   if(!a.lw && a.n <= (size_t)nsm * 2 * 32 * kPairs) {
     auto pair = S.g_ntris ? k_radiance_pair<HV_SW | HV_MESH> : k_radiance_pair<HV_SW>;
-    const cudaError_t e = cudaFuncSetAttribute(pair, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pair_bytes());
+    const cudaError_t e = allow_shared((const void*)pair, device);
     if(e != cudaSuccess) return e;
     pair<<<(unsigned)nsm, 64 * kPairs, pair_bytes(), st>>>(S, a);
     return cudaGetLastError();

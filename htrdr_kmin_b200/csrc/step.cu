@@ -9,6 +9,8 @@
 #include <algorithm>
 #include <map>
 #include <memory>
+#include <mutex>
+#include <set>
 
 namespace hg {
 
@@ -362,7 +364,7 @@ step_shape(Fn kern, const PTables& T, uint32_t* threads, uint32_t blocks_per_sm,
   *in_smem = tables <= 96 * 1024;
   *smem = (own ? own : step_event_bytes(*threads)) + (*in_smem ? tables : 0);
   if(*smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem);
+    const cudaError_t e = allow_shared((const void*)kern, device);
     if(e != cudaSuccess) return e;
   }
   int nsm = 0, per_sm = 0;
@@ -374,6 +376,23 @@ step_shape(Fn kern, const PTables& T, uint32_t* threads, uint32_t blocks_per_sm,
 }
 
 }  // namespace
+
+cudaError_t
+allow_shared(const void* kern, int device)
+{
+  static std::mutex mtx;
+  static std::set<std::pair<const void*, int>> allowed;
+  std::lock_guard<std::mutex> lock(mtx);
+  if(allowed.count({kern, device})) return cudaSuccess;
+  cudaFuncAttributes attr;
+  int most = 0;
+  cudaError_t e = cudaFuncGetAttributes(&attr, kern);
+  if(e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+  if(e == cudaSuccess)
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)attr.sharedSizeBytes);
+  if(e == cudaSuccess) allowed.insert({kern, device});
+  return e;
+}
 
 /* The buffer of the last paths of a run (17 MB), one a host thread and device */
 StepBufs&

@@ -367,7 +367,8 @@ batched_impl(htrdr_gpu_batch_item* items, size_t n, const htrdr_gpu_tuning* tuni
   cudaEventRecord(e3, st);
   unsigned long long c[6] = {0, 0, 0, 0, 0, 0};
   if(ok) ok = cuda_ok(cudaMemcpyAsync(c, P.B->d_cnt.ptr, sizeof(c), cudaMemcpyDeviceToHost, st), "D2H");
-  if(ok) ok = cuda_ok(cudaStreamSynchronize(st), "sync");
+  /* also after an error: the launches before it use the thread's buffers */
+  ok = cuda_ok(cudaStreamSynchronize(st), "sync") && ok;
   if(ok) {
     float k = 0, t = 0;
     cudaEventElapsedTime(&k, e1, e2);

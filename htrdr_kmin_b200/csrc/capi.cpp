@@ -90,7 +90,8 @@ draw_map_impl(htrdr_gpu_scene* scn, const htrdr_gpu_request* req,
   cudaEventRecord(e3, st);
   unsigned long long c[6] = {0, 0, 0, 0, 0, 0};
   if(ok) ok = cuda_ok(cudaMemcpyAsync(c, ws.cnt.ptr, sizeof(c), cudaMemcpyDeviceToHost, st), "D2H");
-  if(ok) ok = cuda_ok(cudaStreamSynchronize(st), "cudaStreamSynchronize");
+  /* also after an error: the launches before it use buffers that the next call reuses */
+  ok = cuda_ok(cudaStreamSynchronize(st), "cudaStreamSynchronize") && ok;
   if(ok && stats) {
     float k = 0, t = 0;
     cudaEventElapsedTime(&k, e1, e2);

@@ -141,7 +141,9 @@ cell_walk(PathTrace& p, const DScene* scenes, bool run)
               const double e = (double)te[j];
               sum = fma(e - a, (double)m[j].x, sum);
               a = e;
-              block = block && m[j].x == m[j].y;
+              /* the same bits: a flagged leaf without extinction (0 and -0) is
+               * larger than its cell */
+              block = block && __float_as_int(m[j].x) == __float_as_int(m[j].y);
             }
             block = block && sum < HG_TMIN_ZERO;
             if(block) {

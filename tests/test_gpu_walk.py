@@ -1,0 +1,57 @@
+"""The walk through single-cell leaves and the kernels' hand-over where the
+scene or the run differs from the usual one, against the plain kernel."""
+import numpy as np
+import pytest
+
+from htrdr_kmin_b200 import scene as S
+
+pytestmark = pytest.mark.gpu
+
+
+def _scene(nx=33, ny=29, nz=12, nbands=2, nquads=2, lw=False, mesh=False, cloud=None, tau=1.0, seed=9):
+    z = S.layers_uniform()
+    lo, hi = (8000.0, 12000.0) if lw else (500.0, 600.0)
+    edges = np.linspace(lo, hi, nbands + 1)
+    nq = np.full(nbands, nquads, dtype=np.uint32)
+    ka, ks, w = (S.gas_lw if lw else S.gas_sw)(z, edges[:-1], edges[1:], nq, seed, (1e-6, 1e-3))
+    lwc = S.lwc_power_law((nz, ny, nx), seed)
+    if cloud is not None:  # liquid water in a corner of the grid only
+        lwc[:, cloud:, :] = 0.0
+        lwc[:, :, cloud:] = 0.0
+    full = lambda v: np.full(nbands, v, np.float32)  # noqa: E731
+    sc = S.Scene(layer_z=z, layer_T=S.temperature_profile(z), band_lo=edges[:-1].copy(), band_hi=edges[1:].copy(),
+                 nquads=nq, quad_w=w, gas_ka=ka, gas_ks=ks, cloud_lwc=lwc, cloud_lower=(0.0, 0.0, 1000.0),
+                 cloud_cell=(80.0, 80.0, 1000.0 / nz), cloud_sigma_ext=full(150.0), cloud_ssa=full(0.99),
+                 cloud_g=full(0.85), repeat_clouds=True, optical_thickness=tau, sun_azimuth=30.0,
+                 sun_elevation=40.0)
+    return S.with_terrain(sc, size=nx * 80.0, n=12, amp=150.0, seed=3, repeat=True) if mesh else sc
+
+
+def _request(mode=S.MODE_XWAVE_SW, width=37, height=21, spp=1, seed=11):
+    lw = mode == S.MODE_XWAVE_LW
+    return S.Request(mode=mode, width=width, height=height, spp=spp,
+                     wlen_range=(8000.0, 12000.0) if lw else (500.0, 600.0),
+                     ref_temperature=290.0 if lw else 5778.0, cam_pos=(800.0, -2500.0, 900.0),
+                     cam_tgt=(800.0, 900.0, 1300.0), fov_deg=60.0, seed=seed)
+
+
+def _plain(api, gs, req):
+    gs.set_engine(api.ENGINE_PLAIN)
+    buf, st = gs.draw_map(req)
+    gs.set_engine(api.ENGINE_PERSISTENT)
+    return buf, st
+
+
+@pytest.mark.parametrize("size", [(37, 21), (220, 115)])
+def test_leaves_without_extinction(gpu_lib, size):
+    """A gas that does not absorb: the absorption trees' leaves outside the
+    cloud are large and hold 0, whose sign still marks them as large."""
+    sc = _scene(cloud=15)
+    sc.gas_ka = np.zeros_like(sc.gas_ka)
+    gs = gpu_lib.GpuScene(sc)
+    req = _request(width=size[0], height=size[1])
+    want, sw = _plain(gpu_lib, gs, req)
+    got, st = gs.draw_map(req)
+    np.testing.assert_allclose(got["L"], want["L"], rtol=1e-12, atol=0)
+    for k in ("segments", "collisions", "nodes", "grid_bytes", "realisations"):
+        assert st[k] == sw[k], k

@@ -557,8 +557,8 @@ def run_serve(args):
 
 def alg_bytes_of(st) -> int:
     """Algorithmic bytes of a launch from its counters: 16 per majorant node
-    fetched, the leaf-grid bytes read (9 per majorant-grid lookup, 4 per
-    node-grid lookup), 8 per tentative collision (its raw-property gather:
+    fetched, the leaf-grid bytes used (8 per cell of a majorant grid, 9 where
+    its leaf is larger, 4 per node-grid lookup), 8 per tentative collision (its raw-property gather:
     cloud cell and gas layer) and 32 per realisation (the read-modify-write
     of its FP64 sums and count)."""
     return 16 * st.nodes + st.grid_bytes + 8 * st.collisions + 32 * st.realisations

@@ -927,7 +927,9 @@ trace_voxel(PathTrace& p, const DScene& S)
                         + (uint64_t)T.c[1] * S.gstride[1] + (uint64_t)T.c[2] * S.gstride[2];
       const float2 mm = __ldg(S.maj_grid + gi);
       L = __ldg(S.lvl_grid + gi);
-      p.c_grid += 9;
+      /* as in cell_walk(): the level is of use where the leaf is larger (it is
+       * asked for before that is known, so as not to wait twice) */
+      p.c_grid += S.maj_flag && L == 0 ? 8 : 9;
       v.x = __float_as_uint(mm.x);
       v.y = __float_as_uint(S.maj_flag ? fabsf(mm.y) : mm.y);
       found = true;

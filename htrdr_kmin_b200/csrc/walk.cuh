@@ -249,7 +249,7 @@ cell_walk(PathTrace& p, const DScene* scenes, bool run)
     ++nulls;
   }
   p.c_seg += n;
-  p.c_grid += 9u * n;
+  p.c_grid += 8u * n;
   T.steps += n;
   T.Ts = ts;
   if(Trans) T.Tmin = tmin;

@@ -55,3 +55,16 @@ def test_leaves_without_extinction(gpu_lib, size):
     np.testing.assert_allclose(got["L"], want["L"], rtol=1e-12, atol=0)
     for k in ("segments", "collisions", "nodes", "grid_bytes", "realisations"):
         assert st[k] == sw[k], k
+
+
+def test_grid_bytes_of_single_cells(gpu_lib):
+    """No leaf larger than a cell (no two cells with the same liquid water, no
+    merging): 8 bytes for each voxel of the cloud."""
+    sc = _scene(nx=32, ny=28, nz=12, tau=0.0)
+    sc.cloud_lwc = np.random.default_rng(1).uniform(1e-4, 1e-3, sc.cloud_lwc.shape).astype(np.float32)
+    gs = gpu_lib.GpuScene(sc)
+    req = _request(width=220, height=115)
+    want, sw = _plain(gpu_lib, gs, req)
+    got, st = gs.draw_map(req)
+    assert 0 < st["grid_bytes"] <= 8 * st["segments"] and st["grid_bytes"] % 8 == 0
+    assert st["grid_bytes"] == sw["grid_bytes"]

@@ -452,6 +452,16 @@ def _percentile(v, q):
     return v[min(len(v) - 1, int(round(q * (len(v) - 1))))] if v else None
 
 
+def pool_tuning(args, api, tuning):
+    """The autotuner's tuning for a server that serves from its pool of paths;
+    a command line's tuning as it is."""
+    if args.tuning:
+        return tuning
+    t = type(tuning).from_buffer_copy(tuning)
+    t.engine = api.ENGINE_WAVEFRONT
+    return t
+
+
 def serve_arrivals(api, items, tuning, arrivals, local: int) -> dict:
     """The request loop with continuous batching fed the requests at the
     given arrival times (s from the first); latency = submit -> map in the
@@ -522,7 +532,8 @@ def run_serve(args):
     for i, (gs, r) in enumerate(items):
         arr[i].scene, arr[i].req, arr[i].layout = gs.handle.value, api.to_request(r), api.layout_for(r)
         arr[i].buffer = dev[i].data_ptr()
-    tuning, batched_ms = api.autotune(arr)  # the server runs the engine that wins
+    tuning, batched_ms = api.autotune(arr)
+    tuning = pool_tuning(args, api, tuning)
     for g in gss:
         g.set_engine(api.ENGINE_PLAIN)
     plain_one = [gs.draw_map(r)[1]["total_ms"] for gs, r in items]
@@ -892,7 +903,7 @@ def main():
         rng = np.random.default_rng(5)
         gaps = rng.exponential(1.0 / rate, size=su.n)
         arrivals = np.cumsum(gaps) - gaps[0]
-        served = serve_arrivals(api, su.items, tuning, arrivals, local)
+        served = serve_arrivals(api, su.items, pool_tuning(args, api, tuning), arrivals, local)
         plain = plain_arrivals(api, su.items, arrivals)
         line["serving"] = {
             "rate_req_s": rate, "arrivals": "Poisson, seeded; all requests within ~1/4 of the "

@@ -405,7 +405,8 @@ HG_API_CATCH("htrdr_gpu_draw_maps_batched_accum_device")
 
 /* Autotuner: times the step loop with every candidate block size on the given
  * items (device buffers) with CUDA events and returns the fastest.  Results do
- * not depend on the tuning. */
+ * not depend on the tuning.  Both names of the step loop's engine run the same
+ * kernels here; the persistent one is also what a graph batch takes. */
 extern "C" HTRDR_GPU_API htrdr_gpu_res_T
 htrdr_gpu_autotune(htrdr_gpu_batch_item* items, size_t n, htrdr_gpu_tuning* best, double* best_ms)
 try {
@@ -414,6 +415,7 @@ try {
   htrdr_gpu_stats st;
   double best_t = 1e300;
   htrdr_gpu_tuning t = items_tuning(items, n, nullptr);
+  t.engine = HTRDR_GPU_ENGINE_PERSISTENT;
   htrdr_gpu_res_T res = batched_impl(items, n, &t, &st, false); /* warm-up */
   if(res != HTRDR_GPU_RES_OK) return res;
   for(uint32_t b : blocks) {

@@ -353,8 +353,9 @@ HTRDR_GPU_API void htrdr_gpu_default_tuning(struct htrdr_gpu_tuning* tuning);
 /* Default tuning of a request mode: the step loop in blocks of 256. */
 HTRDR_GPU_API void htrdr_gpu_mode_tuning(int mode, struct htrdr_gpu_tuning* tuning);
 /* Autotuner: times the step loop's candidate block sizes on `items' (device
- * buffers) and returns the fastest; the rendered values do not depend on the
- * tuning. */
+ * buffers) and returns the fastest, for any entry point (its engine is
+ * _PERSISTENT; a server given _WAVEFRONT instead serves from the pool); the
+ * rendered values do not depend on the tuning. */
 HTRDR_GPU_API htrdr_gpu_res_T
 htrdr_gpu_autotune(struct htrdr_gpu_batch_item* items, size_t n, struct htrdr_gpu_tuning* best,
                    double* best_ms);

@@ -68,3 +68,63 @@ def test_grid_bytes_of_single_cells(gpu_lib):
     got, st = gs.draw_map(req)
     assert 0 < st["grid_bytes"] <= 8 * st["segments"] and st["grid_bytes"] % 8 == 0
     assert st["grid_bytes"] == sw["grid_bytes"]
+
+
+def _exact(api, gs, req, buf):
+    """One realisation a pixel: the map holds the plain kernel's weights."""
+    w = gs.realisation_weights(req, 0, req.width * req.height).ravel()
+    assert np.count_nonzero(w) > w.size // 8
+    np.testing.assert_allclose(buf["L"].ravel(), w, rtol=1e-12, atol=0)
+
+
+# the pair kernel alone; the step loop, its last paths in the pair kernel
+@pytest.mark.parametrize("size", [(37, 21), (220, 115)])
+def test_mesh_and_its_last_paths(gpu_lib, size):
+    gs = gpu_lib.GpuScene(_scene(mesh=True))
+    req = _request(width=size[0], height=size[1])
+    buf, st = gs.draw_map(req)
+    assert st["failures"] == 0
+    _exact(gpu_lib, gs, req, buf)
+
+
+@pytest.mark.parametrize("mesh", [False, True])
+def test_mixed_kinds_and_their_last_paths(gpu_lib, mesh):
+    """Shortwave and longwave requests in one queue, more than the pair
+    kernel's lanes, in an order that the queue does not keep."""
+    sw, lw = gpu_lib.GpuScene(_scene(mesh=mesh)), gpu_lib.GpuScene(_scene(lw=True), 0b100)
+    items = [(lw, _request(S.MODE_XWAVE_LW, 90, 70, seed=1)), (sw, _request(S.MODE_XWAVE_SW, 150, 90, seed=2)),
+             (lw, _request(S.MODE_XWAVE_LW, 11, 9, seed=3)), (sw, _request(S.MODE_XWAVE_SW, 101, 99, seed=4))]
+    assert sum(r.width * r.height for _, r in items) > 18944
+    bufs, st = gpu_lib.draw_maps_batched(items)
+    assert st["failures"] == 0
+    for (gs, req), buf in zip(items, bufs):
+        _exact(gpu_lib, gs, req, buf)
+
+
+@pytest.mark.parametrize("grid", ["nodes", "none"])
+def test_scenes_without_a_majorant_grid(gpu_lib, grid):
+    """A scene whose majorant grid (9 bytes a cell and tree) is more than half
+    of the free memory gets the node grid (4 bytes), or none: its maps are
+    those of the same scene created with room for all."""
+    import torch
+    kw = dict(nx=128, ny=128, nz=32, nbands=8, nquads=4, cloud=20)  # 96 trees: 453 and 201 MB
+    sc = _scene(**kw)
+    roomy = gpu_lib.GpuScene(sc)
+    free = torch.cuda.mem_get_info()[0]
+    room = (650 if grid == "nodes" else 330) << 20
+    hog = torch.empty(free - room, dtype=torch.uint8, device="cuda:0")
+    try:
+        gs = gpu_lib.GpuScene(sc)
+        cells = 128 * 128 * 32 * 96
+        # without any grid, no ranks of the trees' grids (4 bytes a tree) either
+        assert roomy.device_bytes - gs.device_bytes == (cells * 5 if grid == "nodes" else cells * 9 + 96 * 4)
+        for size in ((37, 21), (220, 115)):
+            req = _request(width=size[0], height=size[1])
+            buf, st = gs.draw_map(req)
+            assert st["failures"] == 0 and (st["grid_bytes"] > 0) == (grid == "nodes")
+            _exact(gpu_lib, roomy, req, buf)
+            _exact(gpu_lib, gs, req, buf)
+        gs.close()
+    finally:
+        del hog
+        torch.cuda.empty_cache()

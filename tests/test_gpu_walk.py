@@ -128,3 +128,26 @@ def test_scenes_without_a_majorant_grid(gpu_lib, grid):
     finally:
         del hog
         torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("grid", ["nodes", "none"])
+def test_longwave_without_a_majorant_grid(gpu_lib, grid):
+    """As above, for longwave paths: two voxels of the cloud a turn."""
+    import torch
+    sc = _scene(nx=128, ny=128, nz=32, nbands=8, nquads=4, cloud=100, tau=30.0, lw=True)  # 96 trees
+    room = (700 if grid == "nodes" else 380) << 20
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - room, dtype=torch.uint8, device="cuda:0")
+    try:
+        gs = gpu_lib.GpuScene(sc)
+        for size in ((37, 21), (220, 115)):
+            req = _request(S.MODE_XWAVE_LW, *size)
+            want, sw = _plain(gpu_lib, gs, req)
+            buf, st = gs.draw_map(req)
+            assert st["failures"] == 0 and (st["grid_bytes"] > 0) == (grid == "nodes")
+            for k in ("segments", "nodes", "collisions", "grid_bytes"):
+                assert st[k] == sw[k], k
+            np.testing.assert_allclose(buf["L"], want["L"], rtol=1e-12, atol=0)
+        gs.close()
+    finally:
+        del hog
+        torch.cuda.empty_cache()

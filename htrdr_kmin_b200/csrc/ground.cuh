@@ -17,6 +17,7 @@
 #include <float.h>
 #include <stdint.h>
 
+#include "bvh_entry.h"
 #include "dscene.h"
 
 #define HG_NO_PRIM 0xFFFFFFFFu
@@ -131,7 +132,7 @@ g_trace_mesh(const DScene& S, float3 o, float3 d, float r0, float r1, uint32_t f
   float best = r1;
   uint32_t best_i = HG_NO_PRIM;
   const float3 inv = make_float3(1.f / d.x, 1.f / d.y, 1.f / d.z);
-  uint2 stack[HG_BVH_STACK]; /* {first << 3 | count, entry distance} */
+  hg::BvhEntry stack[HG_BVH_STACK];
   int sp = 0;
   float t0;
   const float4 ra = __ldg(S.g_bvh), rb = __ldg(S.g_bvh + 1);
@@ -148,7 +149,7 @@ g_trace_mesh(const DScene& S, float3 o, float3 d, float r0, float r1, uint32_t f
       const uint32_t rf = __float_as_uint(ha.w), rc = __float_as_uint(hb.w);
       const bool left = l && (!r || tl <= tr);
       if(l && r && sp < HG_BVH_STACK)
-        stack[sp++] = make_uint2(left ? rf << 3 | rc : lf << 3 | lc, __float_as_uint(left ? tr : tl));
+        stack[sp++] = hg::bvh_entry(left ? rf : lf, left ? rc : lc, __float_as_uint(left ? tr : tl));
       down = l || r;
       if(down) {
         first = left ? lf : rf;
@@ -175,13 +176,13 @@ g_trace_mesh(const DScene& S, float3 o, float3 d, float r0, float r1, uint32_t f
       }
     }
     /* the nearest way back up that may still hold a closer hit */
-    uint2 n;
+    hg::BvhEntry n;
     do {
       if(sp == 0) goto done;
       n = stack[--sp];
-    } while(__uint_as_float(n.y) > best + 1e-4f * fmaxf(fabsf(best), 1.f));
-    first = n.x >> 3;
-    count = n.x & 7u;
+    } while(__uint_as_float(hg::bvh_enter_bits(n)) > best + 1e-4f * fmaxf(fabsf(best), 1.f));
+    first = n.first;
+    count = hg::bvh_count(n);
   }
 done:
   if(best_i != HG_NO_PRIM) {

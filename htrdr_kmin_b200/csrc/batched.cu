@@ -91,7 +91,6 @@ cudaError_t
 launch_workqueue(const PTables& T0, const htrdr_gpu_tuning& tun, int device, cudaStream_t st, bool may_keep)
 {
   PTables T = T0;
-  T.chunk = tun.queue_chunk;
   T.regroup_period = tun.regroup_period;
   return tun.engine == HTRDR_GPU_ENGINE_SORTED
     ? launch_sorted(T, tun.block_size, tun.blocks_per_sm, device, st)

@@ -188,7 +188,7 @@ struct PTables {
   uint64_t total;
   unsigned long long* next; /* queue head (zeroed before the launch) */
   void* cnt;                /* Counters (zeroed before the launch) */
-  uint32_t chunk, regroup_period;
+  uint32_t regroup_period;
   uint32_t variant = HV_ALL; /* kernel variant (HV_* bits): the scenes' ground and the requests' kinds */
 };
 /* Kernel variant of a launch over these scenes and requests */

@@ -228,7 +228,6 @@ htrdr_gpu_server::launch_round(Slot& s, const std::vector<SReq*>& act)
   T.total = offsets.back();
   T.cnt = s.cnt.ptr;
   T.next = (unsigned long long*)((char*)s.cnt.ptr + 64);
-  T.chunk = cfg.tuning.queue_chunk;
   T.regroup_period = cfg.tuning.regroup_period;
   ok = ok && cuda_ok(cudaEventRecord(s.e0, s.st), "event")
           && cuda_ok(launch_workqueue(T, cfg.tuning, cfg.device, s.st, false), "k_step")
@@ -504,7 +503,6 @@ htrdr_gpu_server::wave_tables_now()
   T.total = w_appended;
   T.cnt = w_cnt.ptr;
   T.next = (unsigned long long*)((char*)w_cnt.ptr + 64);
-  T.chunk = cfg.tuning.queue_chunk;
   T.regroup_period = cfg.tuning.regroup_period;
   return T;
 }
@@ -526,7 +524,7 @@ htrdr_gpu_server::loop_wave()
 
   /* read-back of one launch: queue head, live paths, finished requests */
   auto process = [&](int b) -> bool {
-    if(!cuda_ok(cudaEventSynchronize(w_ev[b]), "chunk")) return false;
+    if(!cuda_ok(cudaEventSynchronize(w_ev[b]), "pool launch")) return false;
     inflight[b] = false;
     float ms = 0;
     if(cudaEventElapsedTime(&ms, w_ta[b], w_tb[b]) == cudaSuccess) busy_ms += ms;

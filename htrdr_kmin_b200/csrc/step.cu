@@ -99,8 +99,8 @@ struct QueueWork {
         if(m & (1u << lane)) {
           const uint32_t i = i0 + __popc(m & ((1u << lane) - 1u));
           if(i < n_in) {
-            /* from the end: first those that the launch before left */
-            load_path(p, e, in + (size_t)(n_in - 1 - i) * kPathV4);
+            /* a pool's from the end: first those that the launch before left */
+            load_path(p, e, in + (size_t)(Kind == WK_POOL ? n_in - 1 - i : i) * kPathV4);
             p.t0 = gtimer() - p.t0; /* saved: busy time so far */
             want = false;
           } else {
@@ -147,22 +147,26 @@ struct QueueWork {
     uint32_t o = 0;
     if(lane == 0 && m) o = atomicAdd(&ctl->n[turn ^ 1u], (uint32_t)__popc(m));
     o = __shfl_sync(HG_FULL, o, 0) + __popc(m & ((1u << lane) - 1u));
-    if(keep && o < room) { /* else: counted, for the host to see */
+    if(keep && (Kind != WK_POOL || o < room)) { /* else: counted, for the host to see */
       p.t0 = gtimer() - p.t0;
       save_path(p, e, out + (size_t)o * kPathV4);
     }
   }
 };
 
-/* Whether this lane stays empty (warp_lanes); the warps are counted across the
- * blocks first, so that a pool of few paths runs on all SMs */
+/* Whether this lane stays empty: few paths are spread over all warps, as a
+ * warp with a single path takes its bounces fastest.  A pool's lanes have their
+ * limit besides (warp_lanes), the warps counted across the blocks first, so
+ * that a pool of few paths runs on all SMs. */
+template <int Kind>
 __device__ __forceinline__ bool
-lane_unused(const PTables& T, uint32_t saved, uint32_t warp, uint32_t warps_per_block, uint64_t room)
+lane_unused(const PTables& T, uint32_t saved, uint32_t warps_per_block, uint32_t room)
 {
   const unsigned long long next = *(volatile unsigned long long*)T.next;
   const unsigned long long left = saved + (T.total > next ? T.total - next : 0ull);
-  return (threadIdx.x & 31u) >= warp_lanes((uint64_t)warp * gridDim.x + blockIdx.x,
-                                           (uint64_t)gridDim.x * warps_per_block, room, left);
+  const unsigned long long warps = (unsigned long long)gridDim.x * warps_per_block;
+  if(Kind != WK_POOL) return (threadIdx.x & 31u) >= (left + warps - 1) / warps;
+  return (threadIdx.x & 31u) >= warp_lanes((uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x, warps, room, left);
 }
 
 template <int Kind>
@@ -180,8 +184,9 @@ queue_work(const PTables& T, StepSums* sums, const StepPool& P, unsigned long lo
     work.out = P.paths[P.turn ^ 1u];
     work.ctl = P.ctl;
     work.turn = P.turn;
-    work.room = P.lanes;
-    work.n_in = work.kReads ? min(P.ctl->n[P.turn], P.lanes) : 0u;
+    work.room = Kind == WK_POOL ? P.lanes : 0u;
+    work.n_in = work.kReads ? P.ctl->n[P.turn] : 0u;
+    if(Kind == WK_POOL) work.n_in = min(work.n_in, P.lanes);
     work.until = until;
     work.fresh = fresh;
     work.saved_left = work.n_in != 0;
@@ -218,8 +223,7 @@ step_block(PTables& T, const StepPool& P, int tables_in_smem)
 {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ StepSums sums;
-  const bool unused = lane_unused(T, QueueWork<Kind>::kReads ? P.ctl->n[P.turn] : 0u, threadIdx.x >> 5,
-                                  blockDim.x >> 5, Kind == WK_POOL ? P.lanes : UINT64_MAX);
+  const bool unused = lane_unused<Kind>(T, QueueWork<Kind>::kReads ? P.ctl->n[P.turn] : 0u, blockDim.x >> 5, P.lanes);
   __shared__ unsigned long long until;
   __shared__ bool fresh;
   if(threadIdx.x == 0) {
@@ -268,7 +272,7 @@ k_pair(PTables T, StepPool P, int tables_in_smem)
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ StepSums sums;
   __shared__ uint32_t live[kPairs];
-  const bool unused = lane_unused(T, P.ctl->n[P.turn], (threadIdx.x >> 5) % kPairs, kPairs, UINT64_MAX);
+  const bool unused = lane_unused<WK_LAST_IN>(T, P.ctl->n[P.turn], kPairs, 0u);
   if(threadIdx.x == 0) sums = StepSums{0, 0, 0, 0, 0};
   PairJob* jobs = (PairJob*)(smem + step_event_bytes(32 * kPairs));
   if(tables_in_smem) tables_to_smem(T, smem + pair_bytes());
@@ -449,7 +453,6 @@ launch_step(const PTables& T, uint32_t block_size, uint32_t blocks_per_sm, int d
     }
     P.paths[0] = (uint4*)B.paths[0].ptr;
     P.turn = 1; /* saves into paths[0] */
-    P.lanes = B.lanes;
     most<<<grid, block_size, smem, st>>>(T, P, in_smem);
     note_launches(1);
     if((e = cudaGetLastError())) return e;

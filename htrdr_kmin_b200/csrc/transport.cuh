@@ -929,7 +929,7 @@ trace_voxel(PathTrace& p, const DScene& S)
       L = __ldg(S.lvl_grid + gi);
       /* as in cell_walk(): the level is of use where the leaf is larger (it is
        * asked for before that is known, so as not to wait twice) */
-      p.c_grid += S.maj_flag && L == 0 ? 8 : 9;
+      p.c_grid += 8u + (L != 0);
       v.x = __float_as_uint(mm.x);
       v.y = __float_as_uint(S.maj_flag ? fabsf(mm.y) : mm.y);
       found = true;

@@ -136,6 +136,7 @@ cell_walk(PathTrace& p, const DScene* scenes, bool run)
 #pragma unroll
             for(int j = 1; j <= kWalkBlock; ++j) m[j] = __ldg(maj + c[j]);
             double a = td, sum = tmin;
+            int differ = 0;
 #pragma unroll
             for(int j = 0; j < kWalkBlock; ++j) {
               const double e = (double)te[j];
@@ -143,9 +144,9 @@ cell_walk(PathTrace& p, const DScene* scenes, bool run)
               a = e;
               /* the same bits: a flagged leaf without extinction (0 and -0) is
                * larger than its cell */
-              block = block && __float_as_int(m[j].x) == __float_as_int(m[j].y);
+              differ |= __float_as_int(m[j].x) ^ __float_as_int(m[j].y);
             }
-            block = block && sum < HG_TMIN_ZERO;
+            block = !differ && sum < HG_TMIN_ZERO;
             if(block) {
               gx = bx; gy = by; gz = bz;
               tx = dx; ty = dy; tz = dz;

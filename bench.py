@@ -884,9 +884,10 @@ def main():
         su.close()
         return
     tuning, src = pick_tuning(args, api, su, args.workload)
+    # DRAM bytes a launch were measured on these workloads; the others are scaled from the small scenes
+    key = {"mix_full": "k_step", "lw_flux": "k_step_lw"}.get(args.workload, "k_step_small")
     fields, gpu_maps, _ = measure(args, api, su, desc, tuning, src, rank, world, dist,
-                                  traffic_key="k_step_lw" if (args.workload == "lw_flux"
-                                                                 and tuning.engine != api.ENGINE_SORTED) else "")
+                                  traffic_key=key if tuning.engine != api.ENGINE_SORTED else "")
 
     line = {"metric": METRIC, "value": fields.pop("value"), "unit": UNIT, "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": fields.pop("ms_per_step"),

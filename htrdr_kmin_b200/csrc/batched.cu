@@ -318,8 +318,10 @@ htrdr_gpu_default_tuning(htrdr_gpu_tuning* t)
 }
 
 /* The step loop for every mode, blocks of 256 (one an SM for shortwave, two
- * for longwave; 128 measured the same).  The other fields matter to the
- * block-sorted engine, to serving (wave_slots) or no longer. */
+ * for longwave; 128 measured the same).  Of the other fields regroup_period
+ * matters to the block-sorted engine and wave_slots to a server's pool; nothing
+ * reads queue_chunk, trace_budget and wave_tail, whose values stay as callers
+ * know them. */
 extern "C" HTRDR_GPU_API void
 htrdr_gpu_mode_tuning(int mode, htrdr_gpu_tuning* t)
 {

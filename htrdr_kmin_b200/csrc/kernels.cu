@@ -385,8 +385,13 @@ launch_radiance(const DScene& S, const RayArgs& a, int device, cudaStream_t st)
   if(!a.n) return cudaSuccess;
   int nsm = 0, per_sm = 0;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
-  /* shortwave rays that fit in its lanes twice go to the pair kernel: 20 000
-   * rays under a cloud 16.5 ms, 24.4 in the step loop */
+  /* shortwave rays that fit in its lanes twice go to the pair kernel.  Both sides
+   * measured under a repeated cloud of 64x64x32 cells (pairs / step loop): 1000
+   * rays 7.5 / 10.8 ms, 18 900 12.8 / 17.1, 20 000 13.0 / 17.0, 37 000 17.4 /
+   * 21.8, 60 000 20.4 / 24.5, 100 000 26.8 / 27.3, 200 000 45.1 / 41.4; with a
+   * droplet albedo of 0.9, a bounded cloud of 32x32x16 and a mesh the sides cross
+   * between 100 000 and 200 000 too.  So the line is on the safe side: the call
+   * takes a quarter longer just above it than just below. */
   if(!a.lw && a.n <= (size_t)nsm * 2 * 32 * kPairs) {
     auto pair = S.g_ntris ? k_radiance_pair<HV_SW | HV_MESH> : k_radiance_pair<HV_SW>;
     const cudaError_t e = allow_shared((const void*)pair, device);

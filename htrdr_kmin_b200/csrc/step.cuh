@@ -14,7 +14,7 @@
  * loop, all lanes of a warp in one phase, and the traces' frequent part apart
  * (cell_walk).  Lanes regrouped at every voxel step instead, in whatever state
  * they are, took 41 us a bounce at the tail of a small image and 72 us at the
- * tail of a flux map; 47 and 128 ms against 14 and 28 ms for the whole calls. */
+ * tail of a flux map; 47 and 128 ms against 12 and 27 ms for the whole calls. */
 #ifndef HTRDR_STEP_CUH
 #define HTRDR_STEP_CUH
 
@@ -24,24 +24,25 @@
 namespace {
 
 /* Registers of the kernels that run the loop.  Shortwave: all of them (8 warps
- * per SM) against 168 (12): 5.1 against 5.6 ms for 1024 realisations, 31
- * against 34 ms for a flux map of 88 000; batches of long walks are as fast
- * with either.  Longwave, whose bounces are short: 128 (16 warps) against 168
- * and 96: 20.2, 21.2 and 21.4 ms for a flux map of 4.2 M realisations. */
+ * per SM) against 168 (12): a batch of 32 images 293 against 341 ms, a flux map
+ * of 88 000 realisations 27.3 against 28.0, a CIE image 15.3 against 15.6.
+ * Longwave, whose bounces are short: 128 (16 warps) against 96, 112 and 168:
+ * 13.9, 15.7, 14.7 and 18.0 ms for a flux map of 4.2 M realisations, 11.1, 12.5,
+ * 11.7 and 12.8 for an image of 2.3 M. */
 __host__ __device__ constexpr int
 step_registers(unsigned v)
 {
   return (v & HV_SW) ? 255 : 128;
 }
 /* A phase's trace goes on until a quarter of the warp's paths is left in it;
- * these go on when the phase comes round again.  1/4, 1/8 and 1/16 measured
- * within 5 %, 1/4 first. */
+ * these go on when the phase comes round again.  1/4, 1/8 and 1/16: a batch of
+ * 32 images 293, 297 and 308 ms, single maps within 2 %. */
 constexpr uint32_t kStepLag = 4;
 /* Idle lanes that make a warp take new work (the sensor and spectral sampling
  * is the longest piece of code, so it waits for a few lanes), and the lanes of
  * a longwave warp that go on scattering without the others.  Measured on the
- * longwave flux map (idle lanes, lanes): 8, 24 19.9 ms; 8, 16 16.9; 16, 12
- * 16.6; 20, 5 18.3. */
+ * longwave flux map and image (idle lanes, lanes): 8, 24 16.0 and 12.7 ms; 8, 16
+ * 13.8 and 11.2; 16, 12 13.9 and 11.1; 20, 5 17.1 and 12.3. */
 __host__ __device__ constexpr uint32_t
 step_refill(unsigned v)
 {
